@@ -7,8 +7,8 @@
 //    parities) of kappa_c * A_cell x_c.  Cells of one colour share no DoF, so
 //    the read-modify-write needs no atomics; 2^d launches give A(kappa) x in a
 //    fixed order (deterministic).
-//  * kappa_smoother_kernel: one patch per CTA, box residual b - A(kappa) x
-//    assembled cell by cell (the patch's 2^d cells), local solve by fast
+//  * kappa_smoother_kernel (2D; 3D: kappa3d.cuh): one patch per CTA, box residual
+//    b - A(kappa) x assembled cell by cell (the patch's 4 cells), local solve by fast
 //    diagonalization of the unit-coefficient patch scaled by the
 //    patch-averaged coefficient per DoF, D^-1/2 FD^-1 D^-1/2 with D_i the
 //    mean kappa of the patch cells containing DoF i (exact on couplings
@@ -253,32 +253,29 @@ __global__ void __launch_bounds__(KappaCfg<DIM, K>::NT)
   }
 }
 
-// kappa smoother: one patch of colour `colour` per CTA
-template <int DIM, int K, typename T>
+// 2D kappa smoother (3D: kappa3d.cuh): one patch of colour `colour` per CTA
+template <int K, typename T>
 struct KSm {
   static constexpr int NP = K + 1, N1 = 2 * K + 1, M = 2 * K - 1;
-  static constexpr int NC = 1 << DIM;  // cells of a patch
-  static constexpr int BOX = DIM == 3 ? N1 * N1 * N1 : N1 * N1;
-  static constexpr int INT = DIM == 3 ? M * M * M : M * M;
-  static constexpr int CELL = DIM == 3 ? NP * NP * NP : NP * NP;
-  static constexpr int NT = DIM == 3 ? 256 : 128;
+  static constexpr int NC = 4;  // cells of a patch
+  static constexpr int BOX = N1 * N1, INT = M * M, CELL = NP * NP;
+  static constexpr int NT = 128;
   // X[BOX] | TA | TB | UA | UB (NC cells each); the local solve reuses UA, UB
   static constexpr int ELEMS = BOX + 4 * NC * CELL;
   static_assert(NC * CELL >= INT, "the local-solve buffers live in the cell buffers");
 };
 
-// kappa patch smoother: one CTA per patch.  The box residual is assembled
-// from the 2^d cells of the patch contracted at once (each 1D stage has a
-// line task per cell and line, so the CTA's threads share all cells' work),
-// the per-cell results are combined per interior node, then the local solve.
-template <int DIM, int K, typename T>
-__global__ void __launch_bounds__(KSm<DIM, K, T>::NT)
-    kappa_smoother_kernel(T *__restrict__ x, const T *__restrict__ b, const T *__restrict__ kappa,
-                          int n, int colour, int nx_c, int ny_c, int64_t sy, int64_t sz, T s,
-                          T fd_scale, T omega)
+// The box residual is assembled from the 4 cells of the patch contracted at
+// once (each 1D stage has a line task per cell and line, so the CTA's threads
+// share all cells' work), the per-cell results are combined per interior
+// node, then the local solve.
+template <int K, typename T>
+__global__ void __launch_bounds__(KSm<K, T>::NT)
+    kappa_smoother_kernel(T *__restrict__ x, const T *__restrict__ b, const T *__restrict__ kappa, int n,
+                          int colour, int nx_c, int64_t sy, T s, T fd_scale, T omega)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
-  using S = KSm<DIM, K, T>;
+  using S = KSm<K, T>;
   constexpr int NP = S::NP, N1 = S::N1, M = S::M, NT = S::NT, NC = S::NC, CELL = S::CELL;
   const DegreeTables<K, T> &tb = c_tables<K, T>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -287,33 +284,23 @@ __global__ void __launch_bounds__(KSm<DIM, K, T>::NT)
   T *TA = X + S::BOX, *TB = TA + NC * CELL, *UA = TB + NC * CELL, *UB = UA + NC * CELL;
   T *Q1 = UA, *Q2 = UB;  // local solve, after the residual is assembled
   const int j = blockIdx.x;
-  const int px = (colour & 1) + 2 * (j % nx_c);
-  const int py = ((colour >> 1) & 1) + 2 * (DIM == 3 ? (j / nx_c) % ny_c : j / nx_c);
-  const int pz = DIM == 3 ? ((colour >> 2) & 1) + 2 * (j / (nx_c * ny_c)) : 0;
-  const int64_t first = int64_t(px) * K + int64_t(py) * K * sy + int64_t(pz) * K * sz;
-  for (int l = threadIdx.x; l < S::BOX; l += NT) {
-    const int lx = l % N1, ly = (l / N1) % N1, lz = DIM == 3 ? l / (N1 * N1) : 0;
-    X[l] = x[first + lx + ly * sy + lz * sz];
-  }
+  const int px = (colour & 1) + 2 * (j % nx_c), py = ((colour >> 1) & 1) + 2 * (j / nx_c);
+  const int64_t first = int64_t(px) * K + int64_t(py) * K * sy;
+  for (int l = threadIdx.x; l < S::BOX; l += NT) X[l] = x[first + l % N1 + (l / N1) * sy];
   T kpat[NC];
 #pragma unroll
-  for (int cc = 0; cc < NC; ++cc) {
-    const int ox = cc & 1, oy = (cc >> 1) & 1, oz = (cc >> 2) & 1;
-    kpat[cc] = kappa[int64_t(px + ox) + int64_t(py + oy) * n + (DIM == 3 ? int64_t(pz + oz) * n * n : 0)];
-  }
+  for (int cc = 0; cc < NC; ++cc) kpat[cc] = kappa[int64_t(px + (cc & 1)) + int64_t(py + (cc >> 1)) * n];
   if (threadIdx.x < NC) {
 #pragma unroll
     for (int cc = 0; cc < NC; ++cc)
       if (cc == threadIdx.x) kps[cc] = kpat[cc];
   }
   __syncthreads();
-  constexpr int LINES = CELL / NP;  // lines of one cell along one direction
-  // x: TA = M_x x_c, TB = L_x x_c, per cell [c][z][y][x]
-  for (int t = threadIdx.x; t < NC * LINES; t += NT) {
-    const int cc = t / LINES, r = t % LINES;
-    const int ox = cc & 1, oy = (cc >> 1) & 1, oz = (cc >> 2) & 1;
-    const int yl = r % NP, zl = DIM == 3 ? r / NP : 0;
-    const T *src = X + (DIM == 3 ? (oz * K + zl) * N1 * N1 : 0) + (oy * K + yl) * N1 + ox * K;
+  // x: TA = M_x x_c, TB = L_x x_c, per cell [c][y][x]
+  for (int t = threadIdx.x; t < NC * NP; t += NT) {
+    const int cc = t / NP, r = t % NP;
+    const int ox = cc & 1, oy = (cc >> 1) & 1;
+    const T *src = X + (oy * K + r) * N1 + ox * K;
     T v[NP];
 #pragma unroll
     for (int q = 0; q < NP; ++q) v[q] = src[q];
@@ -331,125 +318,65 @@ __global__ void __launch_bounds__(KSm<DIM, K, T>::NT)
     }
   }
   __syncthreads();
-  if constexpr (DIM == 3) {
-    // y: UA = M_y TA, UB = L_y TA + M_y TB
-    for (int t = threadIdx.x; t < NC * LINES; t += NT) {
-      const int cc = t / LINES, r = t % LINES;
-      const int xl = r % NP, zl = r / NP;
-      const T *sa = TA + cc * CELL + zl * NP * NP + xl, *sb = TB + cc * CELL + zl * NP * NP + xl;
-      T va[NP], vb[NP];
+  // y: UA = s kappa_c (L_y TA + M_y TB)
+  for (int t = threadIdx.x; t < NC * NP; t += NT) {
+    const int cc = t / NP, xl = t % NP;
+    const T *sa = TA + cc * CELL + xl, *sb = TB + cc * CELL + xl;
+    T va[NP], vb[NP];
 #pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        va[q] = sa[q * NP];
-        vb[q] = sb[q * NP];
-      }
-      T *da = UA + cc * CELL + zl * NP * NP + xl, *db = UB + cc * CELL + zl * NP * NP + xl;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        T a = T(0), c = T(0);
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-          a += tb.cmass[i * NP + q] * va[q];
-          c += tb.clap[i * NP + q] * va[q] + tb.cmass[i * NP + q] * vb[q];
-        }
-        da[i * NP] = a;
-        db[i * NP] = c;
-      }
+    for (int q = 0; q < NP; ++q) {
+      va[q] = sa[q * NP];
+      vb[q] = sb[q * NP];
     }
-    __syncthreads();
-    // z: TA = s kappa_c (L_z UA + M_z UB) = the cell's A_c x_c
-    for (int t = threadIdx.x; t < NC * LINES; t += NT) {
-      const int cc = t / LINES, r = t % LINES;
-      const T *sa = UA + cc * CELL + r, *sb = UB + cc * CELL + r;
-      T va[NP], vb[NP];
+    const T sk = s * kps[cc];
+    T *d = UA + cc * CELL + xl;
 #pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        va[q] = sa[q * NP * NP];
-        vb[q] = sb[q * NP * NP];
-      }
-      const T sk = s * kps[cc];
-      T *d = TA + cc * CELL + r;
+    for (int i = 0; i < NP; ++i) {
+      T a = T(0);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        T a = T(0);
-#pragma unroll
-        for (int q = 0; q < NP; ++q) a += tb.clap[i * NP + q] * va[q] + tb.cmass[i * NP + q] * vb[q];
-        d[i * NP * NP] = sk * a;
-      }
-    }
-  } else {
-    // y: UA = s kappa_c (L_y TA + M_y TB)
-    for (int t = threadIdx.x; t < NC * LINES; t += NT) {
-      const int cc = t / LINES, xl = t % LINES;
-      const T *sa = TA + cc * CELL + xl, *sb = TB + cc * CELL + xl;
-      T va[NP], vb[NP];
-#pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        va[q] = sa[q * NP];
-        vb[q] = sb[q * NP];
-      }
-      const T sk = s * kps[cc];
-      T *d = UA + cc * CELL + xl;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        T a = T(0);
-#pragma unroll
-        for (int q = 0; q < NP; ++q) a += tb.clap[i * NP + q] * va[q] + tb.cmass[i * NP + q] * vb[q];
-        d[i * NP] = sk * a;
-      }
+      for (int q = 0; q < NP; ++q) a += tb.clap[i * NP + q] * va[q] + tb.cmass[i * NP + q] * vb[q];
+      d[i * NP] = sk * a;
     }
   }
   __syncthreads();
-  const T *OUT = DIM == 3 ? TA : UA;
-  // D^-1/2 of interior DoF l: mean kappa of the patch cells containing it
-  auto dinv_sqrt = [&](int l) -> T {
-    const int c3[3] = {l % M + 1, (l / M) % M + 1, DIM == 3 ? l / (M * M) + 1 : 0};
-    T acc = T(0);
-    int cnt = 0;
-#pragma unroll
-    for (int cc = 0; cc < NC; ++cc) {
-      bool in = true;
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) {
-        const int o = (cc >> d) & 1;
-        in = in && !(o == 0 && c3[d] > K) && !(o == 1 && c3[d] < K);
-      }
-      if (in) {
-        acc += kpat[cc];
-        ++cnt;
-      }
-    }
-    return T(1) / sqrt(acc / T(cnt));
-  };
-  // (A(kappa) x)_l of interior node l: the sum over the patch cells containing it
-  auto ax_node = [&](int l) -> T {
-    const int c3[3] = {l % M + 1, (l / M) % M + 1, DIM == 3 ? l / (M * M) + 1 : 0};
-    T acc = T(0);
+  // visit(cell, node index in the cell) for the patch cells that hold interior DoF l
+  auto cells_of = [&](int l, auto &&visit) {
+    const int c2[2] = {l % M + 1, l / M + 1};
 #pragma unroll
     for (int cc = 0; cc < NC; ++cc) {
       bool in = true;
       int li = 0, mul = 1;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) {
+      for (int d = 0; d < 2; ++d) {
         const int o = (cc >> d) & 1;
-        in = in && !(o == 0 && c3[d] > K) && !(o == 1 && c3[d] < K);
-        li += (c3[d] - o * K) * mul;
+        in = in && !(o == 0 && c2[d] > K) && !(o == 1 && c2[d] < K);
+        li += (c2[d] - o * K) * mul;
         mul *= NP;
       }
-      if (in) acc += OUT[cc * CELL + li];
+      if (in) visit(cc, li);
     }
-    return acc;
+  };
+  // D^-1/2 of interior DoF l: mean kappa of the patch cells containing it
+  auto dinv_sqrt = [&](int l) -> T {
+    T acc = T(0);
+    int cnt = 0;
+    cells_of(l, [&](int cc, int) {
+      acc += kpat[cc];
+      ++cnt;
+    });
+    return T(1) / sqrt(acc / T(cnt));
   };
   // interior residual r = D^-1/2 (b_I - (A(kappa) x)_I); Q1 overlaps the cell
-  // results in 2D, so all of them are combined before Q1 is written
+  // results, so all of them are combined before Q1 is written
   constexpr int RU = (S::INT + NT - 1) / NT;
   T rloc[RU];
 #pragma unroll
   for (int u = 0; u < RU; ++u) {
     const int l = threadIdx.x + u * NT;
     if (l < S::INT) {
-      const int lx = l % M + 1, ly = (l / M) % M + 1, lz = DIM == 3 ? l / (M * M) + 1 : 0;
-      rloc[u] = (b[first + lx + ly * sy + lz * sz] - ax_node(l)) * dinv_sqrt(l);
+      T ax = T(0);
+      cells_of(l, [&](int cc, int li) { ax += UA[cc * CELL + li]; });
+      rloc[u] = (b[first + l % M + 1 + (l / M + 1) * sy] - ax) * dinv_sqrt(l);
     }
   }
   __syncthreads();
@@ -461,17 +388,11 @@ __global__ void __launch_bounds__(KSm<DIM, K, T>::NT)
   __syncthreads();
   // fast diagonalization: S^T along each direction, scale, S back (ping-pong Q1/Q2)
   T *src = Q1, *dst = Q2;
-  for (int pass = 0; pass < 2 * DIM; ++pass) {
-    const int dir = pass % DIM;
-    const bool tr = pass < DIM;
-    const int stride = dir == 0 ? 1 : dir == 1 ? M : M * M;
-    const int lines = S::INT / M;
-    for (int l = threadIdx.x; l < lines; l += NT) {
-      // base index of line l along dir
-      int bidx;
-      if (dir == 0) bidx = l * M;
-      else if (dir == 1) bidx = (l / M) * M * M + l % M;
-      else bidx = l;
+  for (int pass = 0; pass < 4; ++pass) {
+    const bool tr = pass < 2;
+    const int stride = (pass & 1) == 0 ? 1 : M;
+    for (int l = threadIdx.x; l < M; l += NT) {
+      const int bidx = (pass & 1) == 0 ? l * M : l;  // base index of line l along the direction
       T v[M], q[M];
 #pragma unroll
       for (int i = 0; i < M; ++i) v[i] = src[bidx + i * stride];
@@ -483,15 +404,10 @@ __global__ void __launch_bounds__(KSm<DIM, K, T>::NT)
           acc += (tr ? tb.evec[jj * M + i] : tb.evec[i * M + jj]) * v[jj];
         q[i] = acc;
       }
-      if (pass == DIM - 1) {
+      if (pass == 1) {
         // divide by the eigenvalue sums (modes), scaled back to physical cells
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-          const int e = bidx + i * stride;
-          const int mx = e % M, my = (e / M) % M, mz = DIM == 3 ? e / (M * M) : 0;
-          const T lam = tb.eval[mx] + tb.eval[my] + (DIM == 3 ? tb.eval[mz] : T(0));
-          q[i] = q[i] * fd_scale / lam;
-        }
+        for (int i = 0; i < M; ++i) q[i] = q[i] * fd_scale / (tb.eval[l] + tb.eval[i]);
       }
 #pragma unroll
       for (int i = 0; i < M; ++i) dst[bidx + i * stride] = q[i];
@@ -502,8 +418,8 @@ __global__ void __launch_bounds__(KSm<DIM, K, T>::NT)
     dst = tmp;
   }
   for (int l = threadIdx.x; l < S::INT; l += NT) {
-    const int lx = l % M + 1, ly = (l / M) % M + 1, lz = DIM == 3 ? l / (M * M) + 1 : 0;
-    x[first + lx + ly * sy + lz * sz] = omega * (X[lx + ly * N1 + lz * N1 * N1] + src[l] * dinv_sqrt(l));
+    const int lx = l % M + 1, ly = l / M + 1;
+    x[first + lx + ly * sy] = omega * (X[lx + ly * N1] + src[l] * dinv_sqrt(l));
   }
 }
 

@@ -7,6 +7,7 @@
 
 #include "assemble.cuh"
 #include "kappa.cuh"
+#include "kappa3d.cuh"
 #include "kernel_table.h"
 #include "laplace.cuh"
 #include "laplace3d_march.cuh"
@@ -66,6 +67,13 @@ cudaError_t upload_one(const DegreeData &D)
   for (int r = 0; r < C; ++r)
     for (int q = 0; q < C; ++q)
       t.evec_p[r * C + q] = Pair<T>::make(t.evec[r * M + q], t.evec[r * M + C + 1 + q]);
+  std::vector<T> rlam(static_cast<size_t>(M) * M * M);
+  for (int z = 0; z < M; ++z)
+    for (int y = 0; y < M; ++y)
+      for (int x = 0; x < M; ++x)
+        rlam[(static_cast<size_t>(z) * M + y) * M + x] = static_cast<T>(1.0 / (D.eval[x] + D.eval[y] + D.eval[z]));
+  const cudaError_t e = cudaMemcpyToSymbol(g_rlam3<K, T>, rlam.data(), sizeof(T) * rlam.size());
+  if (e != cudaSuccess) return e;
   return cudaMemcpyToSymbol(c_tables<K, T>, &t, sizeof(t));
 }
 
@@ -127,12 +135,12 @@ cudaError_t set_attributes()
   TPS_SET((restrict_xy_kernel<K, T, XYOut::AddInterior>), (restrict_smem<T>()));
   TPS_SET((restrict_xy_kernel<K, T, XYOut::SetInterior>), (restrict_smem<T>()));
   TPS_SET((restrict_xy_kernel<K, T, XYOut::SetAll>), (restrict_smem<T>()));
-  TPS_SET((kappa_smoother_kernel<2, K, T>), (sizeof(T) * KSm<2, K, T>::ELEMS));
+  TPS_SET((kappa_smoother_kernel<K, T>), (sizeof(T) * KSm<K, T>::ELEMS));
   TPS_SET((patch_residual_kernel<2, K, T>), (sizeof(T) * PVar<2, K>::RES_ELEMS));
   TPS_SET((patch_residual_kernel<3, K, T>), (sizeof(T) * PVar<3, K>::RES_ELEMS));
   TPS_SET((patch_solve_kernel<2, K, T>), (sizeof(T) * PVar<2, K>::SOLVE_ELEMS));
   TPS_SET((patch_solve_kernel<3, K, T>), (sizeof(T) * PVar<3, K>::SOLVE_ELEMS));
-  TPS_SET((kappa_smoother_kernel<3, K, T>), (sizeof(T) * KSm<3, K, T>::ELEMS));
+  TPS_SET((kappa_smoother3d_kernel<K, T>), (Ks3<K, T>::BYTES));
 #if TPS_DEGREE >= 2
 #if TPS_DEGREE >= 5
   // degrees 5..7: the per-patch kernel; 2..4: the patch GEMM below
@@ -652,9 +660,14 @@ cudaError_t kappa_smoother(const LevelGeomH &g, const VecLayout &l, void *x, con
   colour_lattice(DIM, g.n, colour, nx, ny, nz, count);
   if (count == 0) return cudaSuccess;
   const double sc = stiffness_scale(DIM, g.h);
-  TPS_LAUNCH((kappa_smoother_kernel<DIM, K, T>), count, KSm<DIM, K, T>::NT, sizeof(T) * KSm<DIM, K, T>::ELEMS, st,
-      static_cast<T *>(x), static_cast<const T *>(b), static_cast<const T *>(kappa), g.n, colour,
-      nx, ny, l.sy, l.sz, static_cast<T>(sc), static_cast<T>(1.0 / sc), static_cast<T>(omega));
+  if constexpr (DIM == 3)
+    TPS_LAUNCH((kappa_smoother3d_kernel<K, T>), count, (Ks3<K, T>::NT), (Ks3<K, T>::BYTES), st,
+        static_cast<T *>(x), static_cast<const T *>(b), static_cast<const T *>(kappa), g.n, colour,
+        nx, ny, l.sy, l.sz, static_cast<T>(sc), static_cast<T>(1.0 / sc), static_cast<T>(omega));
+  else
+    TPS_LAUNCH((kappa_smoother_kernel<K, T>), count, (KSm<K, T>::NT), (sizeof(T) * KSm<K, T>::ELEMS), st,
+        static_cast<T *>(x), static_cast<const T *>(b), static_cast<const T *>(kappa), g.n, colour, nx, l.sy,
+        static_cast<T>(sc), static_cast<T>(1.0 / sc), static_cast<T>(omega));
   return cudaGetLastError();
 }
 

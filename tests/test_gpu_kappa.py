@@ -47,6 +47,28 @@ def test_kappa_level_ops(cuda, oracle, dim, k, n, dtype, tol):
     assert relerr(x.cpu().numpy(), ref) < tol
 
 
+@pytest.mark.parametrize("k,n", [(1, 5), (1, 8), (2, 3), (4, 2), (5, 4), (6, 2), (7, 3)])
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+def test_kappa_smoother_3d_degrees(cuda, oracle, k, n, dtype, tol):
+    """Both colour orders of the 3D sweep at every degree, on meshes whose
+    colours hold one patch, none, or an uneven number; the tolerance is the
+    level operations' above (12 to 30 rounded sums of up to 15 terms per DoF)."""
+    if (n * k - 1) ** 3 > 4096:  # the dense coarse solve's limit: a mesh of two levels or more
+        n = 2 * ((n + 1) // 2)
+    kap = kappa_field(3, n, 11)
+    P = tps.PoissonProblem(3, k, n, kappa=kap)
+    rng = np.random.default_rng(12)
+    npdt = np.float64 if dtype == torch.float64 else np.float32
+    x0, b = rng.uniform(-1, 1, P.n_dofs()).astype(npdt), rng.uniform(-1, 1, P.n_dofs()).astype(npdt)
+    for reverse in (False, True):
+        ref = oracle.smoother_step(3, k, n, x0, b, kappa=kap, reverse=reverse)
+        x = torch.tensor(x0, device="cuda")
+        tps.PatchSmoother(P).step(x, torch.tensor(b, device="cuda"), reverse=reverse)
+        torch.cuda.synchronize()
+        assert relerr(x.cpu().numpy(), ref) < tol, reverse
+    P.close()
+
+
 @pytest.mark.parametrize("dim,k,n", [(2, 2, 8), (3, 2, 6), (3, 3, 4)])
 def test_kappa_vcycle_and_cg(cuda, oracle, dim, k, n):
     kap = kappa_field(dim, n, 3)
