@@ -11,7 +11,7 @@
 #include "kernel_table.h"
 #include "laplace.cuh"
 #include "laplace3d_march.cuh"
-#include "smoother.cuh"
+#include "smoother2d.cuh"
 #include "smoother3d.cuh"
 #include "smoother3d_gemm.cuh"
 #include "smoother3d_pair.cuh"
@@ -72,16 +72,20 @@ cudaError_t upload_one(const DegreeData &D)
     for (int y = 0; y < M; ++y)
       for (int x = 0; x < M; ++x)
         rlam[(static_cast<size_t>(z) * M + y) * M + x] = static_cast<T>(1.0 / (D.eval[x] + D.eval[y] + D.eval[z]));
-  const cudaError_t e = cudaMemcpyToSymbol(g_rlam3<K, T>, rlam.data(), sizeof(T) * rlam.size());
+  cudaError_t e = cudaMemcpyToSymbol(g_rlam3<K, T>, rlam.data(), sizeof(T) * rlam.size());
+  if (e != cudaSuccess) return e;
+  std::vector<T> rows(2 * N1 * M), rlam2(M * M);
+  for (int j = 0; j < N1; ++j)
+    for (int r = 0; r < M; ++r) {
+      rows[j * M + r] = static_cast<T>(D.pmass[(r + 1) * N1 + j]);
+      rows[(N1 + j) * M + r] = static_cast<T>(D.plap[(r + 1) * N1 + j]);
+    }
+  for (int y = 0; y < M; ++y)
+    for (int x = 0; x < M; ++x) rlam2[y * M + x] = static_cast<T>(1.0 / (D.eval[y] + D.eval[x]));
+  e = cudaMemcpyToSymbol(g_prows2<K, T>, rows.data(), sizeof(T) * rows.size());
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_rlam2<K, T>, rlam2.data(), sizeof(T) * rlam2.size());
   if (e != cudaSuccess) return e;
   return cudaMemcpyToSymbol(c_tables<K, T>, &t, sizeof(t));
-}
-
-template <int DIM, typename T>
-size_t smoother_smem()
-{
-  using S = SmootherShape<DIM, K>;
-  return sizeof(T) * S::PPB * S::PER_PATCH;
 }
 
 template <int DIM, typename T>
@@ -106,7 +110,7 @@ cudaError_t set_attributes()
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                            static_cast<int>(bytes));                                    \
   if (e != cudaSuccess) return e;
-  TPS_SET((smoother_colour_kernel<2, K, T>), (smoother_smem<2, T>()));
+  TPS_SET((smoother2d_kernel<K, T>), (Sm2<K, T>::MAX_WARPS * Sm2<K, T>::WARP_BYTES));
   TPS_SET((smoother3d_kernel<K, T, true, sm3_variant_ppb<K, T, 0>()>), (Sm3<K, T, sm3_variant_ppb<K, T, 0>()>::BYTES));
   TPS_SET((smoother3d_kernel<K, T, true, sm3_variant_ppb<K, T, 1>()>), (Sm3<K, T, sm3_variant_ppb<K, T, 1>()>::BYTES));
   TPS_SET((smoother3d_kernel<K, T, true, sm3_variant_ppb<K, T, 2>()>), (Sm3<K, T, sm3_variant_ppb<K, T, 2>()>::BYTES));
@@ -343,13 +347,29 @@ cudaError_t smoother(const LevelGeomH &g, const VecLayout &l, void *x, const voi
   const double sc = stiffness_scale(DIM, g.h);
   const int cx = colour & 1, cy = (colour >> 1) & 1, cz = (colour >> 2) & 1;
   if constexpr (DIM == 2) {
-    using S = SmootherShape<DIM, K>;
-    (void)zero_x;  // the 2D kernel always reads x (x == 0 gives the same sweep)
+    using S = Sm2<K, T>;
+    (void)zero_x;  // only the ring of a box is read (x == 0 gives the same sweep)
+    (void)variant;
     (void)maps;
     (void)err;
-    TPS_LAUNCH((smoother_colour_kernel<DIM, K, T>), ceil_div(count, S::PPB), S::NT, smoother_smem<DIM, T>(), s,
-        static_cast<T *>(x), static_cast<const T *>(b), l.sy, l.sz, nx, ny, count, cx, cy, cz,
-        static_cast<T>(sc), static_cast<T>(1.0 / sc), static_cast<T>(omega));
+    (void)cz;
+    Sm2Args a;
+    a.nx_c = nx;
+    a.count = count;
+    a.cx = cx;
+    a.cy = cy;
+    a.sy = l.sy;
+    magic_div(static_cast<uint32_t>(nx), a.mx, a.sx);
+    // one warp per CTA until the warps cover the SMs four times, then four;
+    // a warp walks over patches once the resident CTAs are used up
+    const int need = static_cast<int>(ceil_div(count, S::P));
+    static const Residency r =
+        residency(smoother2d_kernel<K, T>, 32 * S::MAX_WARPS, S::MAX_WARPS * S::WARP_BYTES);
+    const int warps = need >= S::MAX_WARPS * r.n_sm ? S::MAX_WARPS : 1;
+    const int ctas = static_cast<int>(ceil_div(need, warps));
+    const int grid = warps == 1 || ctas < r.per_sm * r.n_sm ? ctas : r.per_sm * r.n_sm;
+    TPS_LAUNCH((smoother2d_kernel<K, T>), grid, 32 * warps, warps * S::WARP_BYTES, s, static_cast<T *>(x),
+        static_cast<const T *>(b), a, static_cast<T>(sc), static_cast<T>(omega / sc));
   } else {
     Sm3Args a;
     a.nx_c = nx;

@@ -1,0 +1,43 @@
+"""GPU tests of single level kernels at the sizes where their launch shapes
+change, against the CPU oracle (the level parity over all degrees is in
+test_gpu_parity.py)."""
+import numpy as np
+import pytest
+import torch
+
+import gputensorproductsmoother_b200 as tps
+
+pytestmark = pytest.mark.gpu
+
+# FP64: sums of at most 4 (2k+1) terms per stage, 6 stages deep; FP32 the same in
+# 24 bits: the level parity's tolerances
+TOL = {torch.float64: 1e-12, torch.float32: 2e-5}
+
+
+def relerr(a, b):
+    a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
+    return np.abs(a - b).max() / max(np.abs(b).max(), 1e-300)
+
+
+def sweep_matches(oracle, dim, k, n, dtype, seed=5, relaxation=1.0):
+    npdt = np.float64 if dtype == torch.float64 else np.float32
+    P = tps.PoissonProblem(dim, k, n, relaxation=relaxation)
+    rng = np.random.default_rng(seed)
+    x0, b = rng.uniform(-1, 1, P.n_dofs()).astype(npdt), rng.uniform(-1, 1, P.n_dofs()).astype(npdt)
+    for zero, reverse in ((False, True), (True, False)):
+        ref = oracle.smoother_step(dim, k, n, x0, b, omega=relaxation, zero_init=zero, reverse=reverse)
+        x = torch.tensor(x0, device="cuda")
+        S = tps.PatchSmoother(P)
+        (S.vmult if zero else S.step)(x, torch.tensor(b, device="cuda"), reverse=reverse)
+        torch.cuda.synchronize()
+        assert relerr(x.cpu().numpy(), ref) < TOL[dtype], (zero, reverse)
+    P.close()
+
+
+# one warp per CTA, four warps per CTA, and more patches than the resident
+# warps hold (Q1: 32 patches a warp); every colour lattice but the first is uneven
+@pytest.mark.parametrize("k,n", [(1, 3), (1, 72), (1, 640), (1, 1536), (2, 5), (2, 160), (3, 224), (5, 3), (5, 96),
+                                 (5, 288), (6, 72), (7, 5), (7, 128)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_smoother_2d_launch_shapes(cuda, oracle, k, n, dtype):
+    sweep_matches(oracle, 2, k, n, dtype, relaxation=0.9)
