@@ -338,6 +338,43 @@ __global__ void from_vcycle_kernel(double *dst, const void *z, int z_kind, PadMa
     dst[i] = load_kind(z, z_kind, pad_index(i, pm));
 }
 
+// dst[pad(i)] = src[i] (TO_PADDED) or dst[i] = src[pad(i)]: four entries per
+// thread and step, their loads in flight together (HBM-bound)
+template <typename T, bool TO_PADDED>
+__device__ __forceinline__ void copy_rows(T *__restrict__ dst, const T *__restrict__ src, PadMap pm, int64_t n)
+{
+  constexpr int U = 4;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x * U;
+  for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x * U + threadIdx.x; i0 < n; i0 += step) {
+    T v[U];
+    int64_t at[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t i = i0 + u * static_cast<int64_t>(blockDim.x);
+      at[u] = i < n ? pad_index(i, pm) : -1;
+      if (at[u] >= 0) v[u] = src[TO_PADDED ? i : at[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (at[u] >= 0) dst[TO_PADDED ? at[u] : i0 + u * static_cast<int64_t>(blockDim.x)] = v[u];
+  }
+}
+
+template <typename T>
+__global__ void pad_rows_kernel(T *dst_a, const T *src_a, T *dst_b, const T *src_b, PadMap pm, int64_t n)
+{
+  griddep_wait();  // programmatic launch: the previous kernel's writes are visible
+  copy_rows<T, true>(dst_a, src_a, pm, n);
+  if (dst_b) copy_rows<T, true>(dst_b, src_b, pm, n);
+}
+
+template <typename T>
+__global__ void unpad_rows_kernel(T *dst, const T *src, PadMap pm, int64_t n)
+{
+  griddep_wait();  // programmatic launch: the previous kernel's writes are visible
+  copy_rows<T, false>(dst, src, pm, n);
+}
+
 // dense coarse solve: su[idx[i]] = sum_j inv[i][j] d[idx[j]], one warp per row
 template <typename T>
 __global__ void coarse_dense_kernel(const T *inv, const int *idx, int n, T *su, const T *d)
@@ -498,6 +535,29 @@ cudaError_t launch_coarse_dense(const void *inv, const int *idx, int n_int, void
     TPS_LAUNCH((coarse_dense_kernel<float>), g, 256, 0, s, static_cast<const float *>(inv), idx, n_int,
                                                  static_cast<float *>(su),
                                                  static_cast<const float *>(d));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pad_rows(void *dst_a, const void *src_a, void *dst_b, const void *src_b, PadMap pm, int64_t n,
+                            int elem_bytes, cudaStream_t s)
+{
+  if (elem_bytes == 8)
+    TPS_LAUNCH((pad_rows_kernel<double>), stream_grid(n, 1024), 256, 0, s, static_cast<double *>(dst_a),
+        static_cast<const double *>(src_a), static_cast<double *>(dst_b), static_cast<const double *>(src_b), pm, n);
+  else
+    TPS_LAUNCH((pad_rows_kernel<float>), stream_grid(n, 1024), 256, 0, s, static_cast<float *>(dst_a),
+        static_cast<const float *>(src_a), static_cast<float *>(dst_b), static_cast<const float *>(src_b), pm, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_unpad_rows(void *dst, const void *src, PadMap pm, int64_t n, int elem_bytes, cudaStream_t s)
+{
+  if (elem_bytes == 8)
+    TPS_LAUNCH((unpad_rows_kernel<double>), stream_grid(n, 1024), 256, 0, s, static_cast<double *>(dst),
+        static_cast<const double *>(src), pm, n);
+  else
+    TPS_LAUNCH((unpad_rows_kernel<float>), stream_grid(n, 1024), 256, 0, s, static_cast<float *>(dst),
+        static_cast<const float *>(src), pm, n);
   return cudaGetLastError();
 }
 

@@ -103,6 +103,11 @@ cudaError_t launch_to_vcycle(void *d, int d_kind, PadMap pm, const double *src, 
                              cudaStream_t s);
 cudaError_t launch_from_vcycle(double *dst, const void *z, int z_kind, PadMap pm, int64_t n,
                                cudaStream_t s);
+// rows of N1 entries between a lexicographic vector and one with padded rows
+// (entries of elem_bytes 4 or 8): dst_a = src_a, and dst_b = src_b unless null
+cudaError_t launch_pad_rows(void *dst_a, const void *src_a, void *dst_b, const void *src_b, PadMap pm, int64_t n,
+                            int elem_bytes, cudaStream_t s);
+cudaError_t launch_unpad_rows(void *dst, const void *src, PadMap pm, int64_t n, int elem_bytes, cudaStream_t s);
 cudaError_t launch_fill(void *dst, int elem_bytes, int64_t n, cudaStream_t s);  // zero
 
 // --- batched solves: device-side control of one graph launch -------------

@@ -225,6 +225,12 @@ struct tps_handle {
   DevBuf var_acc[2];    // additive step: the summed patch solves
   int sm_kind = TPS_SMOOTHER_FUSED;  // V-cycle smoothing on levels >= 1
   double add_omega = 0.0;            // additive damping (0: 1/2^dim)
+  // tps_smoother_step on caller vectors (3D): row-padded copies of x and b of
+  // the finest-level size and their TMA views per level, [FP64, FP32]
+  DevBuf stage_x[2], stage_b[2];
+  std::vector<SmootherMaps> stage_maps[2];
+  cudaEvent_t stage_done[2] = {nullptr, nullptr};  // end of the last use, and its stream
+  cudaStream_t stage_stream[2] = {nullptr, nullptr};
   DevBuf dense_inv[2];  // Exact variant: reference-cell interior patch inverse [FP64, FP32]
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -239,6 +245,7 @@ struct tps_handle {
       if (pipe_in[i]) cudaEventDestroy(pipe_in[i]);
       if (pipe_done[i]) cudaEventDestroy(pipe_done[i]);
       if (pipe_out[i]) cudaEventDestroy(pipe_out[i]);
+      if (stage_done[i]) cudaEventDestroy(stage_done[i]);
     }
   }
   const LevelGeomH &fine() const { return lv.back(); }
@@ -352,12 +359,23 @@ VecLayout lex_layout(const tps_handle *h, int level)
   return VecLayout{N1, N1, int64_t(N1) * N1};
 }
 
+// rows padded to a 16-byte pitch in 3D, as TMA views need them
+VecLayout padded_layout(const tps_handle *h, int level, size_t elem_bytes)
+{
+  VecLayout lay = lex_layout(h, level);
+  const int align = static_cast<int>(16 / elem_bytes);
+  if (h->dim == 3) {
+    lay.sy = (lay.N1 + align - 1) / align * align;
+    lay.sz = lay.sy * lay.N1;
+  }
+  return lay;
+}
+
 VcycleVectors &vcycle_vectors(tps_handle *h, int p)
 {
   VcycleVectors &V = h->vc[p];
   if (V.ready) return V;
   const size_t es = p == 0 ? sizeof(double) : sizeof(float);
-  const int align = static_cast<int>(16 / es);
   V.d.clear();
   V.su.clear();
   V.t.clear();
@@ -367,10 +385,7 @@ VcycleVectors &vcycle_vectors(tps_handle *h, int p)
   if (!h->err_flag.p) h->err_flag.alloc(sizeof(int));
   for (int l = 0; l < h->n_levels; ++l) {
     const LevelGeomH &g = h->lv[l];
-    VecLayout lay;
-    lay.N1 = g.N1;
-    lay.sy = h->dim == 3 ? (g.N1 + align - 1) / align * align : g.N1;
-    lay.sz = lay.sy * g.N1;
+    const VecLayout lay = padded_layout(h, l, es);
     const size_t n = static_cast<size_t>(h->dim == 3 ? lay.sz * g.N1 : lay.sy * g.N1);
     V.layout.push_back(lay);
     V.d.emplace_back(new DevBuf);
@@ -1001,6 +1016,84 @@ void autotune_levels(tps_handle *h, int p, cudaStream_t s)
   TPS_CUDA(cudaMemsetAsync(V.su.back()->p, 0, V.su.back()->bytes, s));
 }
 
+// The row-padded copies of tps_smoother_step's vectors and their TMA views,
+// allocated at the finest level's size by the first call that wants them (so
+// captured calls keep valid pointers).  False where there is no memory for
+// them, or the stream is capturing (which allows no allocation) before they
+// exist: the sweep then reads the caller's vectors.
+bool stage_vectors(tps_handle *h, int p, cudaStream_t s)
+{
+  if (!h->stage_maps[p].empty()) return true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  const size_t es = p == 0 ? sizeof(double) : sizeof(float);
+  const VecLayout top = padded_layout(h, h->n_levels - 1, es);
+  const size_t bytes = es * static_cast<size_t>(top.sz) * top.N1;
+  try {
+    if (!h->stage_done[p]) TPS_CUDA(cudaEventCreateWithFlags(&h->stage_done[p], cudaEventDisableTiming));
+    if (!h->stage_x[p].p) h->stage_x[p].alloc(bytes);
+    if (!h->stage_b[p].p) h->stage_b[p].alloc(bytes);
+    TPS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // alloc's fill is done before any stream writes
+  } catch (const ApiError &e) {
+    if (e.code != TPS_ERR_ALLOC) throw;
+    h->stage_x[p].release();
+    h->stage_b[p].release();
+    cudaGetLastError();
+    return false;
+  }
+  std::vector<SmootherMaps> maps(h->n_levels);
+  for (int l = 0; l < h->n_levels; ++l)
+    TPS_CUDA(h->kt->encode_maps[p](padded_layout(h, l, es), h->stage_x[p].p, h->stage_b[p].p, &maps[l]));
+  h->stage_maps[p] = std::move(maps);
+  return true;
+}
+
+// tps_smoother_step on caller vectors by way of row-padded copies
+void staged_smoother_step(tps_handle *h, int level, int p, void *x, const void *b, bool zero_init, bool reverse,
+                          cudaStream_t s)
+{
+  const int es = p == 0 ? 8 : 4;
+  const int64_t N = h->lv[level].N;
+  const VecLayout lay = padded_layout(h, level, es);
+  const PadMap pm = make_padmap(lay.N1, lay.sy);
+  void *px = h->stage_x[p].p, *pb = h->stage_b[p].p;
+  // the copies are shared by all calls of the handle: a call on another
+  // stream waits for the last one (calls inside a capture are ordered by it)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool free_running = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  if (!free_running) cudaGetLastError();
+  if (free_running && s != h->stage_stream[p]) TPS_CUDA(cudaStreamWaitEvent(s, h->stage_done[p], 0));
+  if (zero_init) {
+    TPS_CUDA(cudaMemsetAsync(px, 0, es * static_cast<size_t>(lay.sz) * lay.N1, s));
+    TPS_CUDA(launch_pad_rows(pb, b, nullptr, nullptr, pm, N, es, s));
+  } else {
+    TPS_CUDA(launch_pad_rows(px, x, pb, b, pm, N, es, s));
+  }
+  smoother_sweep(h, level, p, lay, px, pb, reverse, zero_init, &h->stage_maps[p][level], s);
+  TPS_CUDA(launch_unpad_rows(x, px, pm, N, es, s));
+  if (free_running) {
+    TPS_CUDA(cudaEventRecord(h->stage_done[p], s));
+    h->stage_stream[p] = s;
+  }
+}
+
+// Whether a level's 3D sweep on caller vectors pays for the copies: their rows
+// have odd pitches, which no TMA view can describe, so the sweep on the
+// vectors themselves is limited to the plain-load kernel of CTA batches.
+// Measured, us per step, copies + TMA kernels / plain loads: Q4 64^3 FP32 545 /
+// 1931, FP64 1075 / 2156; Q4 16^3 FP32 38 / 65; Q4 4^3 FP32 34 / 58; Q3 8^3 FP64
+// 40 / 52; Q7 4^3 FP64 93 / 119; Q2 32^3 FP32 40 / 46, FP64 46 / 52; Q1 64^3
+// FP32 71 / 82, FP64 66 / 73; but Q2 8^3 FP64 38 / 32 and Q1 32^3 FP64 51 / 42.
+// Two cells per direction have one patch, one launch without the copies.
+bool stage_pays(const tps_handle *h, int level)
+{
+  if (h->dim != 3 || h->has_kappa || h->lv[level].n < 3) return false;
+  return h->k >= 3 || h->lv[level].N >= 200000;
+}
+
 // tps_smoother_step with TPS_TF32 on caller vectors (FP32, lexicographic):
 // the sweep runs on the padded, TMA-addressable V-cycle vectors of the level
 void tc_smoother_step(tps_handle *h, int level, void *x, const void *b, bool zero_init, bool reverse, int passes,
@@ -1337,6 +1430,10 @@ int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *
       return;
     }
     const int p = dt_index(dtype);
+    if (stage_pays(h, level) && stage_vectors(h, p, s)) {
+      staged_smoother_step(h, level, p, x, b, zero_init != 0, reverse != 0, s);
+      return;
+    }
     if (zero_init) TPS_CUDA(cudaMemsetAsync(x, 0, (p == 0 ? 8 : 4) * g.N, s));
     smoother_sweep(h, level, p, lex_layout(h, level), x, b, reverse != 0, zero_init != 0, nullptr, s);
   });

@@ -79,7 +79,12 @@ int tps_laplace_vmult(tps_handle *h, int level, int dtype, void *dst, const void
 
 /* PatchSmoother::vmult / step (include/patch_smoother.cuh:155-292): one 2^d-coloured
  * multiplicative vertex-patch sweep x <- S(x, b); zero_init=1 is vmult (x := 0 first).
- * reverse=1 runs the colours in reverse order (symmetric post-smoothing). */
+ * reverse=1 runs the colours in reverse order (symmetric post-smoothing).
+ * 3D sweeps at degree >= 3 or of at least 2e5 DoFs work on row-padded copies
+ * of x and b: the first such call of a precision allocates two vectors of the
+ * finest level's size, which the handle keeps (without memory for them, or
+ * first called inside a stream capture, the sweep reads x and b in place;
+ * same results). */
 int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *b,
                       int zero_init, int reverse, void *stream);
 

@@ -41,3 +41,51 @@ def sweep_matches(oracle, dim, k, n, dtype, seed=5, relaxation=1.0):
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 def test_smoother_2d_launch_shapes(cuda, oracle, k, n, dtype):
     sweep_matches(oracle, 2, k, n, dtype, relaxation=0.9)
+
+
+# the sweep on row-padded copies of the caller's vectors: one and several
+# levels sharing the copies, the smallest level that takes them, rows that
+# need 0..3 entries of padding
+@pytest.mark.parametrize("k,n", [(3, 3), (3, 8), (4, 4), (5, 6), (6, 4), (7, 3), (2, 32), (1, 64)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_smoother_3d_caller_vectors(cuda, oracle, k, n, dtype):
+    if (n * k - 1) ** 3 > 4096 and n % 2:
+        n += 1
+    sweep_matches(oracle, 3, k, n, dtype, relaxation=0.9)
+
+
+def test_smoother_3d_copies_serve_every_level_and_stream(cuda, oracle):
+    """One handle: sweeps of two levels in turn on two streams, without a host
+    wait between them, give each level's sweep; the memory-starved handle
+    sweeps in place with the same result."""
+    k, n = 4, 8
+    P = tps.PoissonProblem(3, k, n)
+    rng = np.random.default_rng(9)
+    xs, bs, ref = {}, {}, {}
+    for lv, nc in ((2, n), (1, n // 2)):
+        x0, b = (rng.uniform(-1, 1, P.n_dofs(lv)) for _ in range(2))
+        xs[lv], bs[lv] = torch.tensor(x0, device="cuda"), torch.tensor(b, device="cuda")
+        ref[lv] = oracle.smoother_step(3, k, nc, oracle.smoother_step(3, k, nc, x0, b), b)
+    start = {lv: x.clone() for lv, x in xs.items()}
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(2):
+        for lv, st in zip(xs, streams):
+            with torch.cuda.stream(st):
+                tps.PatchSmoother(P, lv).step(xs[lv], bs[lv])
+    torch.cuda.synchronize()
+    for lv in xs:
+        assert relerr(xs[lv].cpu().numpy(), ref[lv]) < 1e-12
+    from gputensorproductsmoother_b200 import _lib as L
+    Q = tps.PoissonProblem(3, k, n)
+    y = start[2].clone()
+    tps.PatchSmoother(Q, 0).step(Q.new_vector(0), Q.new_vector(0))  # the error flag exists
+    L.lib().tps_inject_alloc_failure(1)
+    tps.PatchSmoother(Q, 2).step(y, bs[2])
+    L.lib().tps_inject_alloc_failure(0)
+    z = start[2].clone()
+    tps.PatchSmoother(Q, 2).step(z, bs[2])
+    torch.cuda.synchronize()
+    assert torch.equal(y, z)
+    P.close()
+    Q.close()
