@@ -42,6 +42,7 @@ struct CGScalars {
   double bb;      // b . b
   int breakdown;  // set when p.Ap <= 0 or a non-finite value appears
   int pad;
+  double *x;      // the solution vector (read here, so that a captured iteration serves any of them)
 };
 
 // dst[i] = (Tout) src[i]; round32 != 0 rounds through FP32 first
@@ -71,6 +72,8 @@ cudaError_t launch_cg_init(const double *r, const double *b, void *d, int d_kind
                            int64_t n, double *partial, cudaStream_t s);
 // finalize: sc.rr = sum, sc.bb = sum
 cudaError_t launch_cg_finalize_init(const double *partial, CGScalars *sc, cudaStream_t s);
+// sc.x = x
+cudaError_t launch_cg_set_x(CGScalars *sc, double *x, cudaStream_t s);
 // p = z, partial(r.z) ; z in V-cycle precision
 cudaError_t launch_cg_first_direction(double *p, const void *z, int z_kind, PadMap pm,
                                       const double *r, int64_t n, double *partial, cudaStream_t s);
@@ -81,8 +84,8 @@ cudaError_t launch_cg_finalize_rz(const double *partial, CGScalars *sc, cudaStre
 cudaError_t launch_cg_alpha_partials(const double *partial, int count, CGScalars *sc, cudaStream_t s);
 cudaError_t launch_cg_alpha(const double *p, const double *q, int64_t n, double *partial,
                             CGScalars *sc, cudaStream_t s);
-// x += alpha p, r -= alpha q, d = conv(r), partial(r.r)
-cudaError_t launch_cg_update_xr(double *x, double *r, const double *p, const double *q, void *d,
+// x += alpha p (x = sc.x), r -= alpha q, d = conv(r), partial(r.r)
+cudaError_t launch_cg_update_xr(double *r, const double *p, const double *q, void *d,
                                 int d_kind, PadMap pm, int64_t n, double *partial,
                                 const CGScalars *sc, cudaStream_t s);
 cudaError_t launch_cg_finalize_rr(const double *partial, CGScalars *sc, cudaStream_t s);
@@ -132,5 +135,27 @@ struct BatchConds {
   cudaGraphConditionalHandle h[kBatchMax];
 };
 cudaError_t launch_batch_select(const int *active, const BatchConds &cond, int n, cudaStream_t s);
+
+// One system's vectors, as the loader sees them.
+struct BatchSystem {
+  double *p, *q;  // receive x (with b's Dirichlet rows) and b
+  CGScalars *sc;
+  const int *err;  // the system's bounded-wait flag (may be null)
+  int64_t n;       // DoFs
+  int N1, dim;
+};
+// The caller's vectors of one solve (kernel parameter).
+struct BatchIo {
+  const double *b[kBatchMax];
+  double *x[kBatchMax];
+};
+// before the graph: x_b = b_b, p = x, q = b, zero scalars, sc.x = x
+cudaError_t launch_batch_load(const BatchSystem *sys, const BatchIo &io, int n, cudaStream_t s);
+// what the host needs of a finished system
+struct BatchResult {
+  double rr, bnorm;
+  int iters, breakdown, err, pad;
+};
+cudaError_t launch_batch_collect(BatchLoop b, const BatchSystem *sys, BatchResult *out, cudaStream_t s);
 
 }  // namespace tps

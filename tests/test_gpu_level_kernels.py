@@ -89,3 +89,51 @@ def test_smoother_3d_copies_serve_every_level_and_stream(cuda, oracle):
     assert torch.equal(y, z)
     P.close()
     Q.close()
+
+
+def test_captured_solves_serve_any_vectors(cuda):
+    """The captured CG iteration and the batch's graph are built once and read
+    the caller's vectors from device memory: repeated solves with new right-hand
+    sides, new and reused solution vectors (in place of b too) and on several
+    streams match handles that never solved before."""
+    def rhs(N1, seed):
+        v = np.random.default_rng(seed).uniform(-1, 1, (N1,) * 3)
+        v[[0, -1]] = v[:, [0, -1]] = v[:, :, [0, -1]] = 0.0
+        return torch.tensor(v.ravel(), device="cuda")
+
+    k, n = 3, 8
+    N1 = n * k + 1
+    P = tps.PoissonProblem(3, k, n)
+    MG = tps.MultigridSolvers(P)
+    systems = [(3, k, n), (3, 2, 6), (2, 3, 16)]
+    B = tps.BatchSolver(systems)
+    keep = []
+    for i in range(4):
+        st = torch.cuda.Stream() if i % 2 else torch.cuda.default_stream()
+        with torch.cuda.stream(st):
+            b = rhs(N1, 60 + i)
+            x, rep = MG.solve_cg(b, rel_tol=1e-10)
+            Q = tps.PoissonProblem(3, k, n)
+            ref, rep_ref = tps.MultigridSolvers(Q).solve_cg(b.clone(), rel_tol=1e-10)
+            assert torch.equal(x, ref) and rep.history == rep_ref.history
+            keep.append((x, ref.clone()))
+            bs = [b, rhs(13, 70 + i), torch.tensor(np.random.default_rng(80 + i).uniform(-1, 1, 49 ** 2), device="cuda")]
+            xs = [torch.zeros_like(v) for v in bs]
+            if i == 3:  # the first system's solution takes the place of its right-hand side
+                xs[0] = bs[0]
+            got, reps = B.solve(bs, x=xs)
+            C = tps.BatchSolver(systems)
+            if i < 3:
+                want, wreps = C.solve(bs)
+                for g, w, r, wr in zip(got, want, reps, wreps):
+                    # autotuned tile depths may differ between two handles: rounding of p.q
+                    assert r.iterations == wr.iterations
+                    assert (g - w).abs().max().item() <= 1e-12 * w.abs().max().item()
+            else:
+                assert all(r.converged for r in reps)
+            C.close()
+            Q.close()
+    for x, ref in keep:
+        assert torch.equal(x, ref)
+    P.close()
+    B.close()
