@@ -80,8 +80,8 @@ struct KernelTable {
                          cudaStream_t);
   cudaError_t (*cell_energy[2])(const LevelGeomH &, const VecLayout &, double *e, const double *u,
                                 const double *lam, cudaStream_t);
-  // b = sum over cells and QGauss(k+1) points of f phi_i JxW, interior rows
-  // (FP64; f at the cells' Gauss points, cells then points lexicographic)
+  // b = sum over cells and QGauss(k+1) points of f phi_i JxW, Dirichlet rows
+  // zero (FP64; f at the cells' Gauss points, cells then points lexicographic)
   cudaError_t (*assemble_rhs[2])(const LevelGeomH &, const VecLayout &, double *b, const double *fq, cudaStream_t);
   // 3D FP64 q = A p (z-marching kernel) with the p.q partial sums of a CG step
   // fused: one per CTA into partial (at most capacity), *ctas = their count

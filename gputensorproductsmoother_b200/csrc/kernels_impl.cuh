@@ -131,6 +131,8 @@ cudaError_t set_attributes()
                            cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
   if constexpr (sizeof(T) == 8) {
+    TPS_SET((assemble_rhs_kernel<2, K>), (Asm<2, K>::BYTES));
+    TPS_SET((assemble_rhs_kernel<3, K>), (Asm<3, K>::BYTES));
     TPS_SET((laplace3d_march_kernel<K, T, OpMode::Vmult, true>), (sizeof(T) * OpMarch<K, T>::ELEMS));
     e = cudaFuncSetAttribute(laplace3d_march_kernel<K, T, OpMode::Vmult, true>,
                              cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -702,7 +704,6 @@ cudaError_t mass(const LevelGeomH &g, const VecLayout &l, double *dst, const dou
   return cell_sweep<DIM, double, true>(g, l, dst, src, nullptr, hd, st);
 }
 
-// b = sum over cells and Gauss points of f phi_i JxW (interior rows; b zeroed first)
 // 3D FP64 q = A p with the CG's p.q partial sums fused (one per CTA into
 // partial, at most `capacity`; *ctas receives their count)
 cudaError_t laplace3d_dot(const LevelGeomH &g, const VecLayout &l, void *dst, const void *src, double *partial,
@@ -727,25 +728,24 @@ int laplace3d_ctas(int n)
   return ceil_div(n, Sz::TX) * ceil_div(n, Sz::TY) * n;
 }
 
+// b = sum over cells and Gauss points of f phi_i JxW (Dirichlet rows zero)
 template <int DIM>
 cudaError_t assemble_rhs(const LevelGeomH &g, const VecLayout &l, double *b, const double *fq, cudaStream_t st)
 {
-  const int64_t n = DIM == 3 ? l.sz * g.N1 : l.sy * g.N1;
-  cudaError_t e = cudaMemsetAsync(b, 0, sizeof(double) * n, st);
-  if (e != cudaSuccess) return e;
+  using A = Asm<DIM, K>;
   double hd = 1.0;
   for (int d = 0; d < DIM; ++d) hd *= g.h;
-  for (int c = 0; c < (1 << DIM); ++c) {
-    const int cx = c & 1, cy = (c >> 1) & 1, cz = (c >> 2) & 1;
-    const int nx = (g.n - cx + 1) / 2, ny = (g.n - cy + 1) / 2, nz = DIM == 3 ? (g.n - cz + 1) / 2 : 1;
-    const int count = nx * ny * nz;
-    if (count == 0) continue;
-    TPS_LAUNCH((assemble_rhs_kernel<DIM, K>), static_cast<unsigned>(ceil_div(count, 128)), 128, 0, st, b, fq, g.n,
-        l.sy, l.sz, cx, cy, cz, nx, ny, count, hd);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+  dim3 grid(ceil_div(g.n, A::TX), ceil_div(g.n, A::TY), 1);
+  int layers = 1;
+  if (DIM == 3) {
+    // about four CTAs per SM of a 148-SM part; a chunk of layers computes one
+    // layer more than it owns (two to sixteen CTAs per SM measured within 10 %)
+    const int chunks = static_cast<int>(ceil_div(4 * 148, int64_t(grid.x) * grid.y));
+    layers = static_cast<int>(ceil_div(g.n, chunks));
+    grid.z = ceil_div(g.n, layers);
   }
-  return cudaSuccess;
+  TPS_LAUNCH((assemble_rhs_kernel<DIM, K>), grid, A::NT, A::BYTES, st, b, fq, g.n, l.sy, l.sz, layers, hd);
+  return cudaGetLastError();
 }
 
 template <int DIM>

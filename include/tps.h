@@ -218,8 +218,8 @@ int tps_mass_vmult(tps_handle *h, double *dst, const double *src, void *stream);
  * holds f at the Gauss points: cells lexicographic (x fastest), then the
  * (k+1)^dim points of the cell lexicographic (x fastest); the Gauss points of
  * [0,1] are those of orc_gauss/QGauss(k+1) mapped to the cell.  b: FP64,
- * lexicographic, n_dofs(level) entries.  Deterministic (cells added colour
- * by colour, no atomics). */
+ * lexicographic, n_dofs(level) entries.  Deterministic (every node gathered by
+ * one thread, no atomics). */
 int tps_assemble_rhs(tps_handle *h, int level, const double *f_quad, double *b, void *stream);
 
 /* Adjoint of the solve u = A(kappa)^{-1} M f for a loss J(u) (no reference

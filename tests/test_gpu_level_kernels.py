@@ -137,3 +137,26 @@ def test_captured_solves_serve_any_vectors(cuda):
         assert torch.equal(x, ref)
     P.close()
     B.close()
+
+
+# one and several tiles per direction with remainders, one and several layer
+# chunks; every entry of b is written (it starts as NaN), Dirichlet rows as zero
+@pytest.mark.parametrize("dim,k,n", [(3, 1, 40), (3, 1, 72), (3, 2, 20), (3, 3, 12), (3, 4, 12), (3, 5, 8), (3, 6, 8),
+                                     (3, 7, 8), (2, 1, 70), (2, 2, 2), (2, 3, 36), (2, 4, 20), (2, 6, 24)])
+def test_assemble_tiles(cuda, oracle, dim, k, n):
+    from gputensorproductsmoother_b200 import _lib as L
+    P = tps.PoissonProblem(dim, k, n)
+    fq = np.random.default_rng(31 * dim + k).uniform(-1, 1, (n ** dim, (k + 1) ** dim))
+    b = torch.full((P.n_dofs(),), float("nan"), dtype=torch.float64, device="cuda")
+    f = torch.tensor(fq, device="cuda")
+    L.check(L.lib().tps_assemble_rhs(P.handle, P.n_levels - 1, f.data_ptr(), b.data_ptr(), None), P.handle)
+    torch.cuda.synchronize()
+    ref = oracle.assemble_rhs(dim, k, n, fq)
+    got = b.cpu().numpy()
+    assert np.isfinite(got).all()
+    # sums of 2^dim (k+1)^dim products in another order
+    assert relerr(got, ref) < 1e-13
+    v = got.reshape((n * k + 1,) * dim)
+    for ax in range(dim):
+        assert not np.take(v, [0, -1], axis=ax).any()
+    P.close()
