@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "blas.cuh"
+#include "coarse_inverse.cuh"
 #include "fe_data.h"
 #include "kernel_table.h"
 
@@ -173,7 +174,7 @@ struct VcycleVectors {
   std::vector<std::unique_ptr<DevBuf>> d, su, t, tmp;  // per level
   std::vector<VecLayout> layout;                       // per level
   std::vector<SmootherMaps> maps;                      // TMA descriptors (x = su, b = d)
-  DevBuf coarse_inv;                                   // dense coarse inverse
+  DevBuf coarse_inv;                                   // dense coarse inverse (FP32; FP64: the handle's)
   DevBuf coarse_idx;                                   // interior DoFs of the coarse level
 };
 
@@ -190,7 +191,9 @@ struct tps_handle {
   // coarse level: single vertex patch (n_coarse == 2) or dense solve
   bool dense_coarse = false;
   int n_int_coarse = 0;
-  std::vector<double> coarse_inv_host;  // n_int^2, FP64
+  DevBuf coarse_inv;                    // n_int^2, FP64
+  DevBuf coarse_work[2];                // its assembly and inversion
+  DevBuf coarse_tab;                    // reference-cell mass and stiffness, the inversion's flag
   std::vector<int> coarse_coord;        // (x, y, z) of each interior coarse DoF
   VcycleVectors vc[2];  // [0] FP64, [1] FP32
   std::vector<int> sm_variant[2];  // per level: 3D smoother patches-per-batch variant (autotuned)
@@ -288,67 +291,51 @@ int guarded(tps_handle *h, F &&f)
   }
 }
 
-// dense interior operator of the coarse level, assembled cell by cell on the
-// host in FP64 (with the coarse-level kappa when present), and its inverse
+// dense interior operator of the coarse level (with the coarse-level kappa
+// when present) and its FP64 inverse, on the device; the handle's inverse is
+// replaced once the new one is known to be good
 void build_dense_coarse(tps_handle *h)
 {
-  const int k = h->k, n = h->n_coarse, N1 = n * k + 1, dim = h->dim;
-  const double hh = 1.0 / n, s = stiffness_scale(dim, hh);
-  const int np = k + 1;
-  std::vector<int> idx1;
-  for (int i = 1; i < N1 - 1; ++i) idx1.push_back(i);
-  const int m1 = static_cast<int>(idx1.size());
+  const int k = h->k, n = h->n_coarse, dim = h->dim, m1 = n * k - 1;
   const int ni = dim == 3 ? m1 * m1 * m1 : m1 * m1;
+  const size_t bytes = sizeof(double) * static_cast<size_t>(ni) * ni, nt = h->D.cmass.size();
+  if (!h->coarse_tab.p) {
+    h->coarse_tab.alloc(sizeof(double) * (2 * nt + 1));
+    double *t = h->coarse_tab.as<double>();
+    TPS_CUDA(cudaMemcpy(t, h->D.cmass.data(), sizeof(double) * nt, cudaMemcpyHostToDevice));
+    TPS_CUDA(cudaMemcpy(t + nt, h->D.clap.data(), sizeof(double) * nt, cudaMemcpyHostToDevice));
+  }
+  for (DevBuf &w : h->coarse_work)
+    if (!w.p) w.alloc(bytes);
+  if (!h->coarse_inv.p) h->coarse_inv.alloc(bytes);
+  double *t = h->coarse_tab.as<double>(), *a = h->coarse_work[0].as<double>();
+  int *bad = reinterpret_cast<int *>(t + 2 * nt);
+  const CoarseOperator op{dim, k, n, t, t + nt, h->has_kappa ? h->kappa_dev[0][0]->as<double>() : nullptr,
+                          stiffness_scale(dim, 1.0 / n)};
+  TPS_CUDA(launch_assemble_coarse(a, op, ni, nullptr));
+  TPS_CUDA(launch_spd_inverse(a, h->coarse_work[1].as<double>(), ni, bad, nullptr));
+  int failed = 0;
+  TPS_CUDA(cudaMemcpy(&failed, bad, sizeof(int), cudaMemcpyDeviceToHost));
+  if (failed) throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
+  TPS_CUDA(cudaMemcpy(h->coarse_inv.p, a, bytes, cudaMemcpyDeviceToDevice));
+  TPS_CUDA(cudaStreamSynchronize(nullptr));  // any stream may read it from here on
+  if (bytes > (size_t(32) << 20))
+    for (DevBuf &w : h->coarse_work) w.release();
   h->n_int_coarse = ni;
-  auto coord = [&](int i, int &x, int &y, int &z) {
-    x = idx1[i % m1];
-    y = idx1[(i / m1) % m1];
-    z = dim == 3 ? idx1[i / (m1 * m1)] : 0;
-  };
-  // interior index of a global coarse DoF (-1 on the boundary)
-  auto interior = [&](int x, int y, int z) -> int {
-    if (x < 1 || x > N1 - 2 || y < 1 || y > N1 - 2) return -1;
-    if (dim == 3 && (z < 1 || z > N1 - 2)) return -1;
-    return (x - 1) + (y - 1) * m1 + (dim == 3 ? (z - 1) * m1 * m1 : 0);
-  };
-  std::vector<double> A(static_cast<size_t>(ni) * ni, 0.0);
-  const int ncell = dim == 3 ? n * n * n : n * n;
-  const int csz = dim == 3 ? np * np * np : np * np;
-  for (int c = 0; c < ncell; ++c) {
-    const int cx = c % n, cy = (c / n) % n, cz = dim == 3 ? c / (n * n) : 0;
-    const double kc = h->has_kappa ? h->kappa_host[0][c] : 1.0;
-    for (int a = 0; a < csz; ++a) {
-      const int ax = a % np, ay = (a / np) % np, az = dim == 3 ? a / (np * np) : 0;
-      const int ia = interior(cx * k + ax, cy * k + ay, cz * k + az);
-      if (ia < 0) continue;
-      for (int b2 = 0; b2 < csz; ++b2) {
-        const int bx = b2 % np, by = (b2 / np) % np, bz = dim == 3 ? b2 / (np * np) : 0;
-        const int ib = interior(cx * k + bx, cy * k + by, cz * k + bz);
-        if (ib < 0) continue;
-        const double mx = h->D.cmass[ax * np + bx], my = h->D.cmass[ay * np + by];
-        const double lx = h->D.clap[ax * np + bx], ly = h->D.clap[ay * np + by];
-        double v;
-        if (dim == 2) {
-          v = ly * mx + my * lx;
-        } else {
-          const double mz = h->D.cmass[az * np + bz], lz = h->D.clap[az * np + bz];
-          v = lz * my * mx + mz * ly * mx + mz * my * lx;
-        }
-        A[static_cast<size_t>(ia) * ni + ib] += kc * s * v;
-      }
-    }
-  }
-  // explicit inverse (coarse systems hold at most a few thousand DoFs)
-  std::vector<double> inv;
-  try {
-    inv = spd_inverse(A, ni);
-  } catch (const std::runtime_error &) {
-    throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
-  }
-  h->coarse_inv_host = std::move(inv);
   h->coarse_coord.resize(3 * static_cast<size_t>(ni));
-  for (int i = 0; i < ni; ++i) coord(i, h->coarse_coord[3 * i], h->coarse_coord[3 * i + 1],
-                                     h->coarse_coord[3 * i + 2]);
+  for (int i = 0; i < ni; ++i) {
+    h->coarse_coord[3 * i] = 1 + i % m1;
+    h->coarse_coord[3 * i + 1] = 1 + (i / m1) % m1;
+    h->coarse_coord[3 * i + 2] = dim == 3 ? 1 + i / (m1 * m1) : 0;
+  }
+}
+
+// the FP32 V-cycle's rounded copy of the dense coarse inverse
+void round_coarse_inverse(tps_handle *h)
+{
+  TPS_CUDA(launch_convert_f64_to_f32(h->vc[1].coarse_inv.as<float>(), h->coarse_inv.as<double>(),
+                                     static_cast<int64_t>(h->n_int_coarse) * h->n_int_coarse, nullptr));
+  TPS_CUDA(cudaStreamSynchronize(nullptr));
 }
 
 VecLayout lex_layout(const tps_handle *h, int level)
@@ -413,16 +400,9 @@ VcycleVectors &vcycle_vectors(tps_handle *h, int p)
     V.coarse_idx.alloc(sizeof(int) * ni);
     TPS_CUDA(cudaMemcpy(V.coarse_idx.p, gidx.data(), sizeof(int) * ni, cudaMemcpyHostToDevice));
   }
-  if (h->dense_coarse) {
-    const size_t n2 = h->coarse_inv_host.size();
-    V.coarse_inv.alloc(es * n2);
-    if (p == 0) {
-      TPS_CUDA(cudaMemcpy(V.coarse_inv.p, h->coarse_inv_host.data(), es * n2, cudaMemcpyHostToDevice));
-    } else {
-      std::vector<float> f(n2);
-      for (size_t i = 0; i < n2; ++i) f[i] = static_cast<float>(h->coarse_inv_host[i]);
-      TPS_CUDA(cudaMemcpy(V.coarse_inv.p, f.data(), es * n2, cudaMemcpyHostToDevice));
-    }
+  if (h->dense_coarse && p == 1) {
+    V.coarse_inv.alloc(sizeof(float) * static_cast<size_t>(h->n_int_coarse) * h->n_int_coarse);
+    round_coarse_inverse(h);
   }
   V.ready = true;
   return V;
@@ -569,7 +549,7 @@ void coarse_solve(tps_handle *h, int p, cudaStream_t s, bool tc)
     // one vertex patch covers every interior DoF: the smoother is an exact solve
     smoother_sweep(h, 0, p, lay, V.su[0]->p, V.d[0]->p, false, true, &V.maps[0], s, tc);
   } else {
-    TPS_CUDA(launch_coarse_dense(V.coarse_inv.p, V.coarse_idx.as<int>(), h->n_int_coarse,
+    TPS_CUDA(launch_coarse_dense(p == 0 ? h->coarse_inv.p : V.coarse_inv.p, V.coarse_idx.as<int>(), h->n_int_coarse,
                                  V.su[0]->p, V.d[0]->p, static_cast<int>(es), s));
   }
 }
@@ -1579,17 +1559,7 @@ int tps_set_kappa(tps_handle *h, const double *kappa, int rebuild_coarse)
     set_kappa_levels(h, kappa);
     if (rebuild_coarse) {
       build_dense_coarse(h);
-      for (int p = 0; p < 2; ++p) {
-        VcycleVectors &V = h->vc[p];
-        if (!V.ready) continue;
-        const size_t n2 = h->coarse_inv_host.size();
-        if (p == 0) {
-          TPS_CUDA(cudaMemcpy(V.coarse_inv.p, h->coarse_inv_host.data(), 8 * n2, cudaMemcpyHostToDevice));
-        } else {
-          std::vector<float> f(h->coarse_inv_host.begin(), h->coarse_inv_host.end());
-          TPS_CUDA(cudaMemcpy(V.coarse_inv.p, f.data(), 4 * n2, cudaMemcpyHostToDevice));
-        }
-      }
+      if (h->vc[1].ready) round_coarse_inverse(h);
     }
     if (h->graph) {  // re-captured on the next solve
       cudaGraphExecDestroy(h->graph);

@@ -160,3 +160,32 @@ def test_assemble_tiles(cuda, oracle, dim, k, n):
     for ax in range(dim):
         assert not np.take(v, [0, -1], axis=ax).any()
     P.close()
+
+
+# one level: the V-cycle is the dense inverse alone.  Sizes below, at and just
+# past the inversion's 32-column blocks and 64-entry tiles, up to its largest
+# ones; cond(A) is at most 4 (2 n k)^2, so that a backward-stable inverse
+# leaves a residual of a few cond * 2^-53
+@pytest.mark.parametrize("dim,k,n", [(2, 1, 2), (2, 1, 3), (2, 2, 3), (2, 1, 7), (2, 1, 9), (2, 4, 2), (3, 1, 5),
+                                     (2, 1, 33), (2, 1, 34), (3, 4, 3), (3, 1, 16), (2, 2, 32)])
+@pytest.mark.parametrize("varying", [False, True])
+def test_dense_coarse_inverse(cuda, dim, k, n, varying):
+    kap = None
+    if varying:
+        kap = np.exp(np.random.default_rng(3).normal(0.0, 0.5, n ** dim))
+    P = tps.PoissonProblem(dim, k, n, n_coarse=n, kappa=kap)
+    b = np.random.default_rng(4).uniform(-1, 1, (n * k + 1,) * dim)
+    for ax in range(dim):
+        np.moveaxis(b, ax, 0)[[0, -1]] = 0.0
+    b = torch.tensor(b.ravel(), device="cuda")
+    for update in range(2 if varying else 1):
+        if update:  # a new coefficient replaces the inverse
+            P.set_kappa(kap[::-1].copy())
+        for precision, tol in (("fp64", 1e-15), ("fp32", 4e-7)):
+            z, r = P.new_vector(), P.new_vector()
+            tps.MultigridSolvers(P).vmult(z, b, precision=precision)
+            tps.LaplaceOperator(P).vmult(r, z)
+            torch.cuda.synchronize()
+            e = ((r - b).norm() / b.norm()).item()
+            assert e < tol * 4 * (2 * n * k) ** 2, (update, precision, e)
+    P.close()
