@@ -33,13 +33,44 @@
 #pragma once
 
 #include "smoother3d.cuh"
+#include "smoother3d_warp.cuh"  // wp_max
 #include "tps_common.cuh"
 
 namespace tps {
 
+// Paddings of the shared arrays, from an exhaustive search for the fewest
+// wavefronts of the warp-wide accesses below (entries; [FP64, FP32][degree]):
+// of TA and TB's y halves and x nodes, of the cell results' rows and planes, and
+// the largest stride of the y-contracted lines.
+struct Ks3Pad {
+  int ty, td, cr, cp, ca;
+};
+template <int K, typename T>
+constexpr Ks3Pad ks3_pad()
+{
+  constexpr Ks3Pad pad[2][8] = {{{},
+                                 {0, 1, 0, 0, 1},
+                                 {0, 2, 4, 4, 9},
+                                 {0, 2, 2, 6, 33},
+                                 {0, 0, 0, 4, 49},
+                                 {0, 1, 4, 13, 81},
+                                 {0, 6, 0, 0, 129},
+                                 {2, 3, 0, 0, 177}},
+                                {{},
+                                 {0, 0, 0, 0, 1},
+                                 {7, 3, 0, 8, 9},
+                                 {0, 5, 0, 4, 25},
+                                 {0, 0, 8, 8, 65},
+                                 {0, 1, 6, 10, 97},
+                                 {0, 14, 4, 12, 129},
+                                 {0, 2, 2, 7, 177}}};
+  return pad[sizeof(T) == 8 ? 0 : 1][K];
+}
+
 template <int K, typename T>
 struct Ks3 {
   static constexpr int NP = K + 1, N1 = 2 * K + 1, M = 2 * K - 1;
+  static constexpr Ks3Pad PAD = ks3_pad<K, T>();
   // a group of G lanes (8 cells x k x-nodes, whole warps) holds YS-th of the y
   // rows; YS groups share a patch where one group's lanes would leave the
   // other stages (2 (k+1) (2k+1) half lines, (2k-1)^2 lines) short of threads
@@ -48,14 +79,15 @@ struct Ks3 {
   static constexpr int NT = G * YS;
   static constexpr int YR = (K + YS - 1) / YS;  // y rows of a group
   static constexpr int BOX = N1 * N1 * N1;
-  // TA, TB: [z][half in y][y from outside][half in x][x from outside]; the
-  // rows of one y half are odd multiples of 8 entries at degree 4, so the two
-  // halves fall on different banks; the centre line is kept in both halves
-  static constexpr int TX = 2 * K, TY = 2 * NP * TX, TSZ = N1 * TY;
-  static constexpr int INT = M * M * M;
-  static constexpr int CSZ = 8 * K * K * K;  // cell results [cell][z][y][x]
-  static constexpr int R1 = TSZ > CSZ ? TSZ : CSZ;
-  static constexpr int RA = R1 > INT ? R1 : INT;
+  // TA, TB: [z][x from outside][half in y][y from outside][half in x]; the
+  // centre line of y is kept in both halves
+  static constexpr int TO = 2 * NP + PAD.ty, TD = 2 * TO + PAD.td, TZ = K * TD, TSZ = N1 * TZ;
+  // cell results on the 2k nodes per direction (the centre once per half): [z][y][x]
+  static constexpr int CR = 2 * K + PAD.cr, CP = 2 * K * CR + PAD.cp, CSZ = 2 * K * CP;
+  // lines contracted in y, written and read across x and y: strides (2k-1, 1,
+  // SX) of (z, y, x); the arrays between the x and z stages are dense
+  static constexpr int SX = PAD.ca, SSZ = (M - 1) * (M + 1 + SX) + 1;
+  static constexpr int RA = wp_max(wp_max(TSZ, CSZ), wp_max(SSZ, M * M * M));
   static constexpr int ELEMS = BOX + 2 * RA;
   static constexpr size_t BYTES = sizeof(T) * ELEMS;
 };
@@ -176,7 +208,7 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
     T v[NP];
 #pragma unroll
     for (int q = 0; q < NP; ++q) v[q] = src[hx ? -q : q];
-    T *da = TA + r * S::TX + hx * K, *db = TB + r * S::TX + hx * K;
+    const int at = z * S::TZ + (ry < NP ? 2 * ry : S::TO + 2 * (ry - NP)) + hx;
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       T a = tb.cmass[(i + 1) * NP] * v[0], c = tb.clap[(i + 1) * NP] * v[0];
@@ -185,26 +217,28 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
         a = fmadd(tb.cmass[(i + 1) * NP + q], v[q], a);
         c = fmadd(tb.clap[(i + 1) * NP + q], v[q], c);
       }
-      da[i] = a;
-      db[i] = c;
+      TA[at + i * S::TD] = a;
+      TB[at + i * S::TD] = c;
     }
   }
   sync();
   // yz stage
   {
-    const int base = (oz ? 2 * K : 0) * S::TY + oy * NP * S::TX + ox * K + d;
-    const int dz = oz ? -S::TY : S::TY;
+    const int base = (oz ? 2 * K : 0) * S::TZ + d * S::TD + oy * S::TO + ox;
+    const int dz = oz ? -S::TZ : S::TZ;
+    T *c0 = TA + (oz ? (2 * K - 1) * S::CP : 0) + (oy ? (2 * K - 1) * S::CR : 0) + (ox ? 2 * K - 1 - d : d);
+    const int cz = oz ? -S::CP : S::CP, cy = oy ? -S::CR : S::CR;
     // the y halves are stored from the outside inward: both step forward
     auto run = [&](auto y0c, auto nyc) {
       constexpr int Y0 = decltype(y0c)::value, NY = decltype(nyc)::value;
       T acc[K][NY];
-      if (cell_lane) ks3_planes<K, T, Y0, NY>(TA + base, TB + base, dz, S::TX, acc);
+      if (cell_lane) ks3_planes<K, T, Y0, NY>(TA + base, TB + base, dz, 2, acc);
       sync();  // TA and TB are read
       if (cell_lane) {
 #pragma unroll
         for (int i = 0; i < K; ++i)
 #pragma unroll
-          for (int q = 0; q < NY; ++q) TA[((o * K + i) * K + Y0 + q) * K + d] = kap * acc[i][q];
+          for (int q = 0; q < NY; ++q) c0[i * cz + (Y0 + q) * cy] = kap * acc[i][q];
       }
     };
     if constexpr (S::YS == 1) {
@@ -217,48 +251,45 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
     }
   }
   sync();
-  // residual line by line, D^-1/2, S^T along x: C (TA) -> TB
+  // residual line by line in y (b is read along x), D^-1/2, S^T along y: C (TA) -> TB
   constexpr int PM = M * M;
   for (int t = tid; t < PM; t += NT) {
-    const int zi = t / M, yi = t - zi * M;  // interior indices
-    const int z = zi + 1, y = yi + 1;
-    const T *bg = b + first + 1 + int64_t(y) * sy + int64_t(z) * sz;
+    const int zi = t / M, xi = t - zi * M;  // interior indices
+    const T *bg = b + first + 1 + xi + sy + int64_t(zi + 1) * sz;
     T r[M];
 #pragma unroll
-    for (int i = 0; i < M; ++i) r[i] = bg[i];
-    // the cells that share the line: below / above the centre plane, or both on it
-    const int zc = z < K ? 0 : z == K ? 1 : 2, yc = y < K ? 0 : y == K ? 1 : 2;
-    const int zd = z <= K ? z - 1 : 2 * K - z - 1, yd = y <= K ? y - 1 : 2 * K - y - 1;
-    for (int az = zc == 2 ? 1 : 0; az <= (zc == 0 ? 0 : 1); ++az)
-      for (int ay = yc == 2 ? 1 : 0; ay <= (yc == 0 ? 0 : 1); ++ay) {
-        const T *c0 = TA + (((az * 2 + ay) * 2) * K + zd) * K * K + yd * K, *c1 = c0 + K * K * K;
+    for (int i = 0; i < M; ++i) r[i] = bg[i * sy32];
+    // the cells that share the line: below / above the centre plane (class 0
+    // and 2), or both on it; their nodes: node index, plus one above the centre
+    const int zc = zi < K - 1 ? 0 : zi == K - 1 ? 1 : 2, xc = xi < K - 1 ? 0 : xi == K - 1 ? 1 : 2;
+    const int zl = zc == 2 ? zi + 1 : zi, xl = xc == 2 ? xi + 1 : xi;
+    for (int az = 0; az <= (zc == 1 ? 1 : 0); ++az)
+      for (int ax = 0; ax <= (xc == 1 ? 1 : 0); ++ax) {
+        const T *c = TA + (zl + az) * S::CP + xl + ax;
 #pragma unroll
-        for (int i = 0; i < K - 1; ++i) {
-          r[i] -= c0[i];
-          r[M - 1 - i] -= c1[i];
-        }
-        r[K - 1] -= c0[K - 1];
-        r[K - 1] -= c1[K - 1];
+        for (int i = 0; i < K; ++i) r[i] -= c[i * S::CR];
+#pragma unroll
+        for (int i = K - 1; i < M; ++i) r[i] -= c[(i + 1) * S::CR];
       }
-    const T *dq = dsq + 3 * yc + 9 * zc;
+    const T *dq = dsq + xc + 9 * zc;
 #pragma unroll
-    for (int i = 0; i < M; ++i) r[i] *= dq[i < K - 1 ? 0 : i == K - 1 ? 1 : 2];
+    for (int i = 0; i < M; ++i) r[i] *= dq[i < K - 1 ? 0 : i == K - 1 ? 3 : 6];
     T q[M];
     evec_apply<K, T, true>(r, q);
-    T *dst = TB + t * M;
+    T *dst = TB + zi * M + xi * S::SX;
 #pragma unroll
     for (int i = 0; i < M; ++i) dst[i] = q[i];
   }
   sync();
-  // S^T along y: TB -> TA
+  // S^T along x: TB -> TA
   for (int t = tid; t < PM; t += NT) {
-    const int zi = t / M, xi = t - zi * M;
+    const int zi = t / M, yi = t - zi * M;
     T v[M], q[M];
 #pragma unroll
-    for (int i = 0; i < M; ++i) v[i] = TB[zi * PM + i * M + xi];
+    for (int i = 0; i < M; ++i) v[i] = TB[zi * M + yi + i * S::SX];
     evec_apply<K, T, true>(v, q);
 #pragma unroll
-    for (int i = 0; i < M; ++i) TA[zi * PM + i * M + xi] = q[i];
+    for (int i = 0; i < M; ++i) TA[t * M + i] = q[i];
   }
   sync();
   // S^T along z, eigenvalue scaling, S along z: TA -> TB
@@ -276,12 +307,13 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
   sync();
   // S along x: TB -> TA
   for (int t = tid; t < PM; t += NT) {
+    const int zi = t / M, yi = t - zi * M;
     T v[M], q[M];
 #pragma unroll
     for (int i = 0; i < M; ++i) v[i] = TB[t * M + i];
     evec_apply<K, T, false>(v, q);
 #pragma unroll
-    for (int i = 0; i < M; ++i) TA[t * M + i] = q[i];
+    for (int i = 0; i < M; ++i) TA[zi * M + yi + i * S::SX] = q[i];
   }
   sync();
   // S along y and the update of x_I
@@ -290,7 +322,7 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
     const int zi = t / M, xi = t - zi * M;
     T v[M], q[M];
 #pragma unroll
-    for (int i = 0; i < M; ++i) v[i] = TA[zi * PM + i * M + xi];
+    for (int i = 0; i < M; ++i) v[i] = TA[zi * M + i + xi * S::SX];
     evec_apply<K, T, false>(v, q);
     const int xc = xi < K - 1 ? 0 : xi == K - 1 ? 1 : 2, zc = zi < K - 1 ? 0 : zi == K - 1 ? 1 : 2;
     const T *dq = dsq + xc + 9 * zc;
