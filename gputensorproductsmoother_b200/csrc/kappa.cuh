@@ -3,9 +3,10 @@
 // path has a unit coefficient (include/laplace_operator.cuh:25-31); these
 // kernels extend the same Q_k discretisation with a per-cell factor.
 //
-//  * cell_apply_kernel: y += sum over the cells of ONE colour (cell index
-//    parities) of kappa_c * A_cell x_c.  Cells of one colour share no DoF, so
-//    the read-modify-write needs no atomics; 2^d launches give A(kappa) x in a
+//  * cell_apply_kernel (the 2D operator, kappa_laplace3d.cuh in 3D; the mass
+//    product): y += sum over the cells of ONE colour (cell index parities) of
+//    kappa_c * A_cell x_c.  Cells of one colour share no DoF, so the
+//    read-modify-write needs no atomics; 2^d launches give A(kappa) x in a
 //    fixed order (deterministic).
 //  * kappa_smoother_kernel (2D; 3D: kappa3d.cuh): one patch per CTA, box residual
 //    b - A(kappa) x assembled cell by cell (the patch's 4 cells), local solve by fast

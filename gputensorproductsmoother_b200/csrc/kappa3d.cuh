@@ -26,12 +26,14 @@
 // multiply-adds per 50 shared loads in the yz stage at degree 4).  The kernel
 // before it ran the stages cell by cell with three shared-memory exchanges and
 // two square roots and divisions per node.  Measured, us per sweep on caller
-// vectors, before / now: Q4 48^3 FP64 3084 / 852, FP32 1416 / 529; Q3 48^3 FP64
-// 1061 / 336; Q2 64^3 FP64 1605 / 325; Q5 32^3 FP64 2274 / 475; Q7 16^3 FP64
-// 793 / 271.  Loading a thread's line of b before the yz stage measured slower
-// (Q4 48^3 FP64 891, Q5 32^3 545: its registers cost resident warps).
+// vectors, before / now: Q4 48^3 FP64 3084 / 618, FP32 1416 / 430; Q4 12^3 FP64
+// 73 / 40; Q3 48^3 FP64 1061 / 263; Q2 64^3 FP64 1605 / 300; Q5 32^3 FP64 2274 / 377;
+// Q7 16^3 FP64 793 / 214.  The x box is copied asynchronously (plain loads one
+// after the other: 752 at Q4 48^3); b copied to shared memory as well, or loaded
+// before the yz stage, measured slower (646 and more: fewer resident patches).
 #pragma once
 
+#include "ptx.cuh"
 #include "smoother3d.cuh"
 #include "smoother3d_warp.cuh"  // wp_max
 #include "tps_common.cuh"
@@ -180,8 +182,9 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
   for (int l = tid; l < S::BOX; l += NT) {
     const int r = l / N1, lx = l - r * N1, lz = r / N1, ly = r - lz * N1;
-    X[l] = x[first + lx + ly * sy32 + int64_t(lz) * sz];
+    cp_async_zfill<sizeof(T)>(X + l, x + first + lx + ly * sy32 + int64_t(lz) * sz, true);
   }
+  cp_async_commit();  // all of a thread's copies in flight at once
   if (tid < 27) {
     const int c3[3] = {tid % 3, (tid / 3) % 3, tid / 9};  // 0 below, 1 on, 2 above
     T acc = T(0);
@@ -198,6 +201,7 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
     }
     dsq[tid] = T(1) / sqrt(acc / T(cnt));
   }
+  cp_async_wait_all();
   sync();
   // x stage: task = (z, half in y, y from outside, half in x)
   for (int t = tid; t < N1 * 2 * NP * 2; t += NT) {

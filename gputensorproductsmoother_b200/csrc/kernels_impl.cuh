@@ -8,6 +8,7 @@
 #include "assemble.cuh"
 #include "kappa.cuh"
 #include "kappa3d.cuh"
+#include "kappa_laplace3d.cuh"
 #include "kernel_table.h"
 #include "laplace.cuh"
 #include "laplace3d_march.cuh"
@@ -147,6 +148,8 @@ cudaError_t set_attributes()
   TPS_SET((patch_solve_kernel<2, K, T>), (sizeof(T) * PVar<2, K>::SOLVE_ELEMS));
   TPS_SET((patch_solve_kernel<3, K, T>), (sizeof(T) * PVar<3, K>::SOLVE_ELEMS));
   TPS_SET((kappa_smoother3d_kernel<K, T>), (Ks3<K, T>::BYTES));
+  TPS_SET((kappa_laplace3d_kernel<K, T, false>), (Kl3<K, T>::BYTES));
+  TPS_SET((kappa_laplace3d_kernel<K, T, true>), (Kl3<K, T>::BYTES));
 #if TPS_DEGREE >= 2
 #if TPS_DEGREE >= 5
   // degrees 5..7: the per-patch kernel; 2..4: the patch GEMM below
@@ -661,14 +664,32 @@ template <int DIM, typename T>
 cudaError_t kappa_laplace(const LevelGeomH &g, const VecLayout &l, void *dst, const void *src,
                           const void *rhs, const void *kappa, int mode, cudaStream_t st)
 {
-  const int64_t n = DIM == 3 ? l.sz * g.N1 : l.sy * g.N1;
+  // Dirichlet rows end at 0 like the unit-coefficient kernel's untouched rows
+  // of zero-initialised work vectors; tps_laplace_vmult then copies src there
+  if constexpr (DIM == 3) {
+    using S = Kl3<K, T>;
+    dim3 grid(ceil_div(g.n, S::TX), ceil_div(g.n, S::TY), 1);
+    // about eight CTAs per SM of a 148-SM part; a chunk of layers computes one
+    // layer more than it owns
+    const int chunks = static_cast<int>(ceil_div(8 * 148, int64_t(grid.x) * grid.y));
+    const int layers = static_cast<int>(ceil_div(g.n, chunks));
+    grid.z = ceil_div(g.n, layers);
+    const T sc = static_cast<T>(stiffness_scale(DIM, g.h));
+    if (mode == 1)
+      TPS_LAUNCH((kappa_laplace3d_kernel<K, T, true>), grid, S::NT, S::BYTES, st, static_cast<T *>(dst),
+          static_cast<const T *>(src), static_cast<const T *>(rhs), static_cast<const T *>(kappa), g.n, l.sy, l.sz,
+          layers, sc);
+    else
+      TPS_LAUNCH((kappa_laplace3d_kernel<K, T, false>), grid, S::NT, S::BYTES, st, static_cast<T *>(dst),
+          static_cast<const T *>(src), nullptr, static_cast<const T *>(kappa), g.n, l.sy, l.sz, layers, sc);
+    return cudaGetLastError();
+  }
+  const int64_t n = l.sy * g.N1;
   cudaError_t e = cudaMemsetAsync(dst, 0, sizeof(T) * n, st);
   if (e != cudaSuccess) return e;
   e = cell_sweep<DIM, T, false>(g, l, static_cast<T *>(dst), static_cast<const T *>(src),
                                 static_cast<const T *>(kappa), stiffness_scale(DIM, g.h), st);
   if (e != cudaSuccess) return e;
-  // Dirichlet rows end at 0 like the unit-coefficient kernel's untouched rows
-  // of zero-initialised work vectors; tps_laplace_vmult then copies src there
   TPS_LAUNCH((finish_residual_kernel<DIM, T>), 1184, 256, 0, st,
       static_cast<T *>(dst), mode == 1 ? static_cast<const T *>(rhs) : nullptr, g.N1, l.sy, l.sz);
   return cudaGetLastError();

@@ -189,3 +189,24 @@ def test_dense_coarse_inverse(cuda, dim, k, n, varying):
             e = ((r - b).norm() / b.norm()).item()
             assert e < tol * 4 * (2 * n * k) ** 2, (update, precision, e)
     P.close()
+
+
+# the varying-coefficient operator and smoother: tiles with remainders, several
+# layer chunks, every degree (the cells' rows are split over two thread groups
+# in FP64 from degree 5 on); padded rows are covered by the V-cycles elsewhere
+@pytest.mark.parametrize("k,n", [(1, 9), (1, 40), (2, 3), (2, 24), (3, 5), (3, 12), (4, 2), (4, 12), (5, 3), (5, 8), (6, 2),
+                                 (6, 8), (7, 2), (7, 4)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_kappa_operator_tiles(cuda, oracle, k, n, dtype):
+    if (tps.split_cells(n)[0] * k - 1) ** 3 > 4096:
+        n = 4
+    npdt = np.float64 if dtype == torch.float64 else np.float32
+    rng = np.random.default_rng(17)
+    kap = np.exp(rng.normal(0.0, 0.5, n ** 3))
+    P = tps.PoissonProblem(3, k, n, kappa=kap)
+    x = rng.uniform(-1, 1, P.n_dofs()).astype(npdt)
+    y = torch.full((P.n_dofs(),), float("nan"), dtype=dtype, device="cuda")
+    tps.LaplaceOperator(P).vmult(y, torch.tensor(x, device="cuda"))
+    torch.cuda.synchronize()
+    assert relerr(y.cpu().numpy(), oracle.laplace_vmult(3, k, n, x, kappa=kap)) < TOL[dtype]
+    P.close()
