@@ -28,6 +28,17 @@ __device__ __forceinline__ void store_kind(void *d, int kind, int64_t i, double 
     static_cast<double *>(d)[i] = v;
 }
 
+// d[i] = v and su[i] = 0 (unless su is null)
+__device__ __forceinline__ void store_d_su(void *d, void *su, int kind, int64_t i, double v)
+{
+  store_kind(d, kind, i, v);
+  if (!su) return;
+  if (kind == 1)
+    static_cast<float *>(su)[i] = 0.f;
+  else
+    static_cast<double *>(su)[i] = 0.0;
+}
+
 __device__ __forceinline__ double load_kind(const void *z, int kind, int64_t i)
 {
   return kind == 1 ? static_cast<double>(static_cast<const float *>(z)[i])
@@ -140,7 +151,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(const double *parti
 }
 
 __global__ void __launch_bounds__(kRedThreads)
-    cg_init_kernel(const double *r, const double *b, void *d, int d_kind, PadMap pm, int64_t n,
+    cg_init_kernel(const double *r, const double *b, void *d, void *su, int d_kind, PadMap pm, int64_t n,
                    double *partial)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
@@ -151,7 +162,7 @@ __global__ void __launch_bounds__(kRedThreads)
     const double ri = r[i], bi = b[i];
     s_rr += ri * ri;
     s_bb += bi * bi;
-    store_kind(d, d_kind, pad_index(i, pm), ri);
+    store_d_su(d, su, d_kind, pad_index(i, pm), ri);
   }
   s_rr = block_sum<kRedThreads>(s_rr, sh);
   s_bb = block_sum<kRedThreads>(s_bb, sh);
@@ -255,7 +266,7 @@ __global__ void __launch_bounds__(kRedThreads)
 
 __global__ void __launch_bounds__(kRedThreads)
     cg_update_xr_kernel(double *__restrict__ r, const double *__restrict__ p, const double *__restrict__ q, void *d,
-                        int d_kind, PadMap pm, int64_t n, double *partial, const CGScalars *sc)
+                        void *su, int d_kind, PadMap pm, int64_t n, double *partial, const CGScalars *sc)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
   __shared__ double sh[32];
@@ -286,7 +297,7 @@ __global__ void __launch_bounds__(kRedThreads)
       const double ri = rv[u] - alpha * qv[u];
       r[j] = ri;
       s += ri * ri;
-      store_kind(d, d_kind, pad_index(j, pm), ri);
+      store_d_su(d, su, d_kind, pad_index(j, pm), ri);
     }
   }
   for (; i < n; i += step) {
@@ -294,7 +305,7 @@ __global__ void __launch_bounds__(kRedThreads)
     const double ri = r[i] - alpha * q[i];
     r[i] = ri;
     s += ri * ri;
-    store_kind(d, d_kind, pad_index(i, pm), ri);
+    store_d_su(d, su, d_kind, pad_index(i, pm), ri);
   }
   s = block_sum<kRedThreads>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
@@ -355,12 +366,12 @@ __global__ void sub_kernel(double *dst, const double *a, const double *b, int64_
     dst[i] = a[i] - b[i];
 }
 
-__global__ void to_vcycle_kernel(void *d, int d_kind, PadMap pm, const double *src, int64_t n)
+__global__ void to_vcycle_kernel(void *d, void *su, int d_kind, PadMap pm, const double *src, int64_t n)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    store_kind(d, d_kind, pad_index(i, pm), src[i]);
+    store_d_su(d, su, d_kind, pad_index(i, pm), src[i]);
 }
 
 __global__ void from_vcycle_kernel(double *dst, const void *z, int z_kind, PadMap pm, int64_t n)
@@ -470,10 +481,10 @@ cudaError_t launch_reduce(const double *partial, int n_dots, double *out, cudaSt
   TPS_LAUNCH((reduce_kernel), n_dots, kRedThreads, 0, s, partial, out);
   return cudaGetLastError();
 }
-cudaError_t launch_cg_init(const double *r, const double *b, void *d, int d_kind, PadMap pm,
+cudaError_t launch_cg_init(const double *r, const double *b, void *d, void *su, int d_kind, PadMap pm,
                            int64_t n, double *partial, cudaStream_t s)
 {
-  TPS_LAUNCH((cg_init_kernel), kRedBlocks, kRedThreads, 0, s, r, b, d, d_kind, pm, n, partial);
+  TPS_LAUNCH((cg_init_kernel), kRedBlocks, kRedThreads, 0, s, r, b, d, su, d_kind, pm, n, partial);
   return cudaGetLastError();
 }
 cudaError_t launch_cg_finalize_init(const double *partial, CGScalars *sc, cudaStream_t s)
@@ -509,11 +520,11 @@ cudaError_t launch_cg_alpha(const double *p, const double *q, int64_t n, double 
   TPS_LAUNCH((finalize_kernel<1, OpAlpha>), 1, kRedThreads, 0, s, partial, sc, OpAlpha{});
   return cudaGetLastError();
 }
-cudaError_t launch_cg_update_xr(double *r, const double *p, const double *q, void *d,
+cudaError_t launch_cg_update_xr(double *r, const double *p, const double *q, void *d, void *su,
                                 int d_kind, PadMap pm, int64_t n, double *partial,
                                 const CGScalars *sc, cudaStream_t s)
 {
-  TPS_LAUNCH((cg_update_xr_kernel), kRedBlocks, kRedThreads, 0, s, r, p, q, d, d_kind, pm, n, partial, sc);
+  TPS_LAUNCH((cg_update_xr_kernel), kRedBlocks, kRedThreads, 0, s, r, p, q, d, su, d_kind, pm, n, partial, sc);
   return cudaGetLastError();
 }
 cudaError_t launch_cg_finalize_rr(const double *partial, CGScalars *sc, cudaStream_t s)
@@ -549,10 +560,10 @@ cudaError_t launch_sub_f64(double *dst, const double *a, const double *b, int64_
   TPS_LAUNCH((sub_kernel), stream_grid(n, 256), 256, 0, s, dst, a, b, n);
   return cudaGetLastError();
 }
-cudaError_t launch_to_vcycle(void *d, int d_kind, PadMap pm, const double *src, int64_t n,
+cudaError_t launch_to_vcycle(void *d, void *su, int d_kind, PadMap pm, const double *src, int64_t n,
                              cudaStream_t s)
 {
-  TPS_LAUNCH((to_vcycle_kernel), stream_grid(n, 256), 256, 0, s, d, d_kind, pm, src, n);
+  TPS_LAUNCH((to_vcycle_kernel), stream_grid(n, 256), 256, 0, s, d, su, d_kind, pm, src, n);
   return cudaGetLastError();
 }
 cudaError_t launch_from_vcycle(double *dst, const void *z, int z_kind, PadMap pm, int64_t n,

@@ -67,8 +67,10 @@ cudaError_t launch_reduce(const double *partial, int n_dots, double *out, cudaSt
 
 // --- fused CG steps (flexible CG, FP64 outer) ---------------------------
 // r = b - A x was formed by the operator; rr, and the V-cycle input d
-// (FP32, FP64, or FP64 rounded through FP32) are produced from r.
-cudaError_t launch_cg_init(const double *r, const double *b, void *d, int d_kind, PadMap pm,
+// (FP32, FP64, or FP64 rounded through FP32) are produced from r.  Every
+// kernel that writes d can zero the V-cycle's solution vector su with it (same
+// type and layout; may be null), which then needs no fill.
+cudaError_t launch_cg_init(const double *r, const double *b, void *d, void *su, int d_kind, PadMap pm,
                            int64_t n, double *partial, cudaStream_t s);
 // finalize: sc.rr = sum, sc.bb = sum
 cudaError_t launch_cg_finalize_init(const double *partial, CGScalars *sc, cudaStream_t s);
@@ -85,7 +87,7 @@ cudaError_t launch_cg_alpha_partials(const double *partial, int count, CGScalars
 cudaError_t launch_cg_alpha(const double *p, const double *q, int64_t n, double *partial,
                             CGScalars *sc, cudaStream_t s);
 // x += alpha p (x = sc.x), r -= alpha q, d = conv(r), partial(r.r)
-cudaError_t launch_cg_update_xr(double *r, const double *p, const double *q, void *d,
+cudaError_t launch_cg_update_xr(double *r, const double *p, const double *q, void *d, void *su,
                                 int d_kind, PadMap pm, int64_t n, double *partial,
                                 const CGScalars *sc, cudaStream_t s);
 cudaError_t launch_cg_finalize_rr(const double *partial, CGScalars *sc, cudaStream_t s);
@@ -102,7 +104,7 @@ cudaError_t launch_scale_f64(double *y, double a, int64_t n, cudaStream_t s);
 cudaError_t launch_sub_f64(double *dst, const double *a, const double *b, int64_t n,
                            cudaStream_t s);  // dst = a - b
 // V-cycle input from an FP64 vector and FP64 output from the V-cycle result
-cudaError_t launch_to_vcycle(void *d, int d_kind, PadMap pm, const double *src, int64_t n,
+cudaError_t launch_to_vcycle(void *d, void *su, int d_kind, PadMap pm, const double *src, int64_t n,
                              cudaStream_t s);
 cudaError_t launch_from_vcycle(double *dst, const void *z, int z_kind, PadMap pm, int64_t n,
                                cudaStream_t s);

@@ -63,10 +63,11 @@ struct KernelTable {
   // fine += P coarse (interior fine DoFs); geometry of the COARSE level
   cudaError_t (*prolong[2][2])(const LevelGeomH &coarse, const VecLayout &lc, const VecLayout &lf,
                                void *fine, const void *coarse_v, void *tmp, cudaStream_t);
-  // coarse (+)= R fine on interior coarse DoFs; geometry of the COARSE level
+  // coarse (+)= R fine on interior coarse DoFs; geometry of the COARSE level;
+  // zero (may be null, not with add): a coarse vector to zero on the interior
   cudaError_t (*restrict_[2][2])(const LevelGeomH &coarse, const VecLayout &lc,
                                  const VecLayout &lf, void *coarse_v, const void *fine, void *tmp,
-                                 int add, cudaStream_t);
+                                 int add, void *zero, cudaStream_t);
   // variable coefficient (kappa per cell, lexicographic cells, precision of the vector):
   // dst = A(kappa) src on interior rows (mode 0) or rhs - A(kappa) src (mode 1)
   cudaError_t (*kappa_laplace[2][2])(const LevelGeomH &, const VecLayout &, void *dst,

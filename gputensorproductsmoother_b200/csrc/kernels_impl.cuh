@@ -605,7 +605,7 @@ cudaError_t prolong_nb(const LevelGeomH &gc, const VecLayout &lc, const VecLayou
 
 template <int DIM, typename T>
 cudaError_t restrict_(const LevelGeomH &gc, const VecLayout &lc, const VecLayout &lf, void *coarse,
-                      const void *fine, void *tmp, int add, cudaStream_t s)
+                      const void *fine, void *tmp, int add, void *zero, cudaStream_t s)
 {
   constexpr int C = XYTile<K>::C;
   const int N1c = gc.N1, N1f = 2 * gc.n * K + 1;
@@ -614,22 +614,23 @@ cudaError_t restrict_(const LevelGeomH &gc, const VecLayout &lc, const VecLayout
   if constexpr (DIM == 2) {
     if (add)
       TPS_LAUNCH((restrict_xy_kernel<K, T, XYOut::AddInterior>), dim3(gxy, gxy, 1), XYTile<K>::NT, smem, s,
-          static_cast<T *>(coarse), static_cast<const T *>(fine), N1c, N1f, lf.sy, 0, lc.sy, 0, 0, 1);
+          static_cast<T *>(coarse), static_cast<const T *>(fine), N1c, N1f, lf.sy, 0, lc.sy, 0, 0, 1, static_cast<T *>(zero));
     else
       TPS_LAUNCH((restrict_xy_kernel<K, T, XYOut::SetInterior>), dim3(gxy, gxy, 1), XYTile<K>::NT, smem, s,
-          static_cast<T *>(coarse), static_cast<const T *>(fine), N1c, N1f, lf.sy, 0, lc.sy, 0, 0, 1);
+          static_cast<T *>(coarse), static_cast<const T *>(fine), N1c, N1f, lf.sy, 0, lc.sy, 0, 0, 1, static_cast<T *>(zero));
   } else {
     const int64_t P = static_cast<int64_t>(N1c) * N1c;
     TPS_LAUNCH((restrict_xy_kernel<K, T, XYOut::SetAll>), dim3(gxy, gxy, N1f), XYTile<K>::NT, smem, s,
-        static_cast<T *>(tmp), static_cast<const T *>(fine), N1c, N1f, lf.sy, lf.sz, N1c, P, 0, N1f);
+        static_cast<T *>(tmp), static_cast<const T *>(fine), N1c, N1f, lf.sy, lf.sz, N1c, P, 0, N1f,
+          nullptr);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (add)
       TPS_LAUNCH((restrict_z_kernel<K, T, true>), dim3(ceil_div(P, 256), gc.n), 256, 0, s,
-          static_cast<T *>(coarse), static_cast<const T *>(tmp), N1c, N1f, lc.sy, lc.sz);
+          static_cast<T *>(coarse), static_cast<const T *>(tmp), N1c, N1f, lc.sy, lc.sz, static_cast<T *>(zero));
     else
       TPS_LAUNCH((restrict_z_kernel<K, T, false>), dim3(ceil_div(P, 256), gc.n), 256, 0, s,
-          static_cast<T *>(coarse), static_cast<const T *>(tmp), N1c, N1f, lc.sy, lc.sz);
+          static_cast<T *>(coarse), static_cast<const T *>(tmp), N1c, N1f, lc.sy, lc.sz, static_cast<T *>(zero));
   }
   return cudaGetLastError();
 }

@@ -160,7 +160,7 @@ extern "C" int tps_restrict_add_noalloc(int dim, int degree, int n_coarse_cells,
   const VecLayout lc{static_cast<int>(N1c), N1c, N1c * N1c};
   const VecLayout lf{static_cast<int>(N1f), N1f, N1f * N1f};
   e = kt->restrict_[dim - 2][dtype == TPS_F64 ? 0 : 1](gc, lc, lf, coarse, fine, scratch, 1,
-                                                       static_cast<cudaStream_t>(stream));
+                                                       nullptr, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(TPS_ERR_CUDA, cudaGetErrorString(e));
   return TPS_OK;
 }

@@ -544,7 +544,7 @@ void coarse_solve(tps_handle *h, int p, cudaStream_t s, bool tc)
   VcycleVectors &V = h->vc[p];
   const size_t es = p == 0 ? sizeof(double) : sizeof(float);
   const VecLayout &lay = V.layout[0];
-  TPS_CUDA(cudaMemsetAsync(V.su[0]->p, 0, es * V.su[0]->bytes / es, s));
+  // either solve writes every interior DoF; the boundary of su stays zero
   if (!h->dense_coarse) {
     // one vertex patch covers every interior DoF: the smoother is an exact solve
     smoother_sweep(h, 0, p, lay, V.su[0]->p, V.d[0]->p, false, true, &V.maps[0], s, tc);
@@ -609,9 +609,11 @@ void level_smooth(tps_handle *h, int level, int p, const VecLayout &lay, void *x
 }
 
 // MultigridSolvers::v_cycle (include/solver.cuh:1952-2001) on precision p:
-// input d[level], output su[level]; tc: FP32 3D sweeps on the tensor cores;
-// zero_init = false continues from the current su[level] (a further cycle of
-// v_cycle(level, n_cycles), include/solver.cuh:798-805)
+// input d[level], output su[level]; tc: FP32 3D sweeps on the tensor cores.
+// su[level] is zero on entry where zero_with names it: whatever writes d[level]
+// zeroes it with the same stores; otherwise it is filled here.
+// zero_init = false continues from the current su[level] instead (a further
+// cycle of v_cycle(level, n_cycles), include/solver.cuh:798-805)
 // Inside the TF32 V-cycle the tensor-core smoother runs a level only where it
 // is faster than the FP32 SIMT kernels: degrees 2..4 (the patch-GEMM kernel)
 // on levels whose colour 0 fills a wave of 128-patch tiles on every SM.
@@ -621,6 +623,18 @@ bool tc_pays(const tps_handle *h, int level)
   if (h->dim != 3 || h->k > 4 || (h->tc_passes == 3 && h->k != 4)) return false;
   const int64_t c = h->lv[level].n / 2;
   return c * c * c >= 128 * static_cast<int64_t>(h->n_sm);
+}
+
+// The V-cycle's solution vector of a level, to be zeroed with the stores that
+// write its right-hand side; null where vcycle_rec fills it itself.  A fill
+// costs its own launch and the overlap of its neighbours' (2D Q2 64^2 solve
+// 1181 us with fills, 1036 without); vectors beyond 16 MB cost more as one more
+// stream of the writing kernel than as a fill (Q4 64^3 solve 10.21 against
+// 10.26 ms).
+void *zero_with(const tps_handle *h, int p, int level)
+{
+  const DevBuf &su = *h->vc[p].su[level];
+  return su.bytes <= (size_t(16) << 20) ? su.p : nullptr;
 }
 
 void vcycle_rec(tps_handle *h, int level, int p, bool symmetric, cudaStream_t s, bool tc,
@@ -639,12 +653,13 @@ void vcycle_rec(tps_handle *h, int level, int p, bool symmetric, cudaStream_t s,
   const LevelGeomH &g = h->lv[level];
   const VecLayout &lay = V.layout[level], &lc = V.layout[level - 1];
   const int di = h->dim - 2;
-  if (zero_init) TPS_CUDA(cudaMemsetAsync(V.su[level]->p, 0, V.su[level]->bytes, s));
+  if (zero_init && !zero_with(h, p, level))
+    TPS_CUDA(cudaMemsetAsync(V.su[level]->p, 0, V.su[level]->bytes, s));
   const bool tcl = tc && tc_pays(h, level);
   level_smooth(h, level, p, lay, V.su[level]->p, V.d[level]->p, false, zero_init, &V.maps[level], s, tcl);
   level_laplace(h, level, p, lay, V.t[level]->p, V.su[level]->p, V.d[level]->p, 1, s);
   TPS_CUDA(h->kt->restrict_[di][p](h->lv[level - 1], lc, lay, V.d[level - 1]->p, V.t[level]->p,
-                                   V.tmp[level]->p, 0, s));
+                                   V.tmp[level]->p, 0, zero_with(h, p, level - 1), s));
   vcycle_rec(h, level - 1, p, symmetric, s, tc);
   TPS_CUDA(h->kt->prolong[di][p](h->lv[level - 1], lc, lay, V.su[level]->p, V.su[level - 1]->p,
                                  V.tmp[level]->p, s));
@@ -781,8 +796,8 @@ void cg_iteration_body(tps_handle *h, int prec, bool symmetric, cudaStream_t s)
   TPS_CUDA(launch_cg_beta(V.su[L]->p, zk, pm, h->q.as<double>(), h->r.as<double>(), N, part, sc, s));
   TPS_CUDA(launch_cg_update_p(h->p.as<double>(), V.su[L]->p, zk, pm, N, sc, s));
   cg_q_alpha(h, lex, s);
-  TPS_CUDA(launch_cg_update_xr(h->r.as<double>(), h->p.as<double>(), h->q.as<double>(),
-                               V.d[L]->p, input_kind(prec), pm, N, part, sc, s));
+  TPS_CUDA(launch_cg_update_xr(h->r.as<double>(), h->p.as<double>(), h->q.as<double>(), V.d[L]->p,
+                               zero_with(h, p, L), input_kind(prec), pm, N, part, sc, s));
   TPS_CUDA(launch_cg_finalize_rr(part, sc, s));
 }
 
@@ -817,7 +832,7 @@ int solve_cg(tps_handle *h, const tps_solve_opts &o, const double *b, double *x,
   TPS_CUDA(cudaMemsetAsync(h->r.p, 0, sizeof(double) * N, s));
   TPS_CUDA(cudaMemsetAsync(h->q.p, 0, sizeof(double) * N, s));
   level_laplace(h, L, 0, lex, h->r.p, x, b, 1, s);
-  TPS_CUDA(launch_cg_init(h->r.as<double>(), b, V.d[L]->p, input_kind(o.precision), pm, N, part, s));
+  TPS_CUDA(launch_cg_init(h->r.as<double>(), b, V.d[L]->p, zero_with(h, p, L), input_kind(o.precision), pm, N, part, s));
   TPS_CUDA(launch_cg_finalize_init(part, sc, s));
   TPS_CUDA(launch_cg_set_x(sc, x, s));
   CGScalars hs{};
@@ -837,8 +852,8 @@ int solve_cg(tps_handle *h, const tps_solve_opts &o, const double *b, double *x,
                                        part, s));
     TPS_CUDA(launch_cg_finalize_rz(part, sc, s));
     cg_q_alpha(h, lex, s);
-    TPS_CUDA(launch_cg_update_xr(h->r.as<double>(), h->p.as<double>(), h->q.as<double>(),
-                                 V.d[L]->p, input_kind(o.precision), pm, N, part, sc, s));
+    TPS_CUDA(launch_cg_update_xr(h->r.as<double>(), h->p.as<double>(), h->q.as<double>(), V.d[L]->p,
+                               zero_with(h, p, L), input_kind(o.precision), pm, N, part, sc, s));
     TPS_CUDA(launch_cg_finalize_rr(part, sc, s));
     it = 1;
     const int key = (o.precision << 1) | (sym ? 1 : 0);
@@ -927,7 +942,7 @@ void apply_vcycle64(tps_handle *h, int precision, bool symmetric, double *dst, c
   const int L = h->n_levels - 1;
   const int64_t N = h->fine().N;
   const PadMap pm = fine_padmap(h, p);
-  TPS_CUDA(launch_to_vcycle(V.d[L]->p, input_kind(precision), pm, src, N, s));
+  TPS_CUDA(launch_to_vcycle(V.d[L]->p, zero_with(h, p, L), input_kind(precision), pm, src, N, s));
   vcycle_rec(h, L, p, symmetric, s, vprec_tc(precision));
   TPS_CUDA(launch_from_vcycle(dst, V.su[L]->p, p == 1 ? 1 : 0, pm, N, s));
 }
@@ -1094,6 +1109,8 @@ void tc_smoother_step(tps_handle *h, int level, void *x, const void *b, bool zer
   TPS_CUDA(cudaMemcpy2DAsync(pb, pitch, b, row, row, rows, cudaMemcpyDeviceToDevice, s));
   smoother_sweep(h, level, 1, l, px, pb, reverse, zero_init, &V.maps[level], s, true);
   TPS_CUDA(cudaMemcpy2DAsync(x, row, px, pitch, row, rows, cudaMemcpyDeviceToDevice, s));
+  // the V-cycle relies on the zero boundary of its solution vectors
+  TPS_CUDA(cudaMemsetAsync(px, 0, V.su[level]->bytes, s));
 }
 
 // MultigridSolvers::solve (include/solver.cuh:1784-1860), see tps_fmg
@@ -1126,7 +1143,7 @@ void fmg(tps_handle *h, int precision, int n_cycles, const double *const *rhs, c
   const int zk = p == 1 ? 1 : 0;
   TPS_CUDA(cudaEventRecord(h->ev0, s));
   // coarse level: coarse solve, then one more smoother step
-  TPS_CUDA(launch_to_vcycle(V.d[0]->p, input_kind(precision), padmap(0), rhs[0], h->lv[0].N, s));
+  TPS_CUDA(launch_to_vcycle(V.d[0]->p, zero_with(h, p, 0), input_kind(precision), padmap(0), rhs[0], h->lv[0].N, s));
   coarse_solve(h, p, s, tc && tc_pays(h, 0));
   smoother_sweep(h, 0, p, V.layout[0], V.su[0]->p, V.d[0]->p, false, false, &V.maps[0], s, tc && tc_pays(h, 0));
   double *sol0 = L == 0 ? x : h->fmg_sol[0]->as<double>();
@@ -1141,7 +1158,7 @@ void fmg(tps_handle *h, int precision, int n_cycles, const double *const *rhs, c
     TPS_CUDA(h->kt->prolong_nb[dim - 2](gc, lex_layout(h, l - 1), lex_layout(h, l), sol, solc, h->fmg_tmp.p, s));
     TPS_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * g.N, s));
     level_laplace(h, l, 0, lex_layout(h, l), res, sol, rhs[l], 1, s);
-    TPS_CUDA(launch_to_vcycle(V.d[l]->p, input_kind(precision), padmap(l), res, g.N, s));
+    TPS_CUDA(launch_to_vcycle(V.d[l]->p, zero_with(h, p, l), input_kind(precision), padmap(l), res, g.N, s));
     for (int c = 0; c < n_cycles; ++c) vcycle_rec(h, l, p, false, s, tc, c == 0);
     TPS_CUDA(launch_from_vcycle(res, V.su[l]->p, zk, padmap(l), g.N, s));
     TPS_CUDA(launch_axpy_f64(sol, 1.0, res, g.N, s));
@@ -1496,7 +1513,7 @@ int tps_restrict_add(tps_handle *h, int from_level, int dtype, void *coarse, con
     VcycleVectors &V = vcycle_vectors(h, p);
     TPS_CUDA(h->kt->restrict_[h->dim - 2][p](h->lv[from_level - 1], lex_layout(h, from_level - 1),
                                              lex_layout(h, from_level), coarse, fine,
-                                             V.tmp[from_level]->p, 1, s));
+                                             V.tmp[from_level]->p, 1, nullptr, s));
   });
 }
 
@@ -2026,7 +2043,7 @@ void batch_init_system(tps_handle *h, int prec, cudaStream_t s)
   VcycleVectors &V = h->vc[p];
   TPS_CUDA(cudaMemsetAsync(h->r.p, 0, sizeof(double) * N, s));
   level_laplace(h, L, 0, lex_layout(h, L), h->r.p, h->p.p, h->q.p, 1, s);
-  TPS_CUDA(launch_cg_init(h->r.as<double>(), h->q.as<double>(), V.d[L]->p, input_kind(prec), fine_padmap(h, p), N,
+  TPS_CUDA(launch_cg_init(h->r.as<double>(), h->q.as<double>(), V.d[L]->p, zero_with(h, p, L), input_kind(prec), fine_padmap(h, p), N,
                           h->partial.as<double>(), s));
   TPS_CUDA(launch_cg_finalize_init(h->partial.as<double>(), h->scalars.as<CGScalars>(), s));
   TPS_CUDA(cudaMemsetAsync(h->p.p, 0, sizeof(double) * N, s));

@@ -199,12 +199,13 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
 
 // xy pass, restriction: fine plane -> coarse plane.  Fine boundary entries
 // are read as zero (weight 0 on Dirichlet DoFs).  zero_plane != 0 writes
-// zeros instead (fine z-boundary planes).
+// zeros instead (fine z-boundary planes).  zero (may be null, SetInterior): a
+// vector of the coarse layout whose interior is zeroed with the same stores.
 template <int K, typename T, XYOut OUT>
 __global__ void __launch_bounds__(XYTile<K>::NT)
     restrict_xy_kernel(T *__restrict__ out, const T *__restrict__ in, int N1c, int N1f,
                        int64_t in_sy, int64_t in_plane, int64_t out_sy, int64_t out_plane,
-                       int plane0, int n_planes_total)
+                       int plane0, int n_planes_total, T *__restrict__ zero)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
   constexpr int C = XYTile<K>::C, NT = XYTile<K>::NT;
@@ -262,7 +263,10 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
       if constexpr (OUT == XYOut::AddInterior) {
         if (interior) outp[gi] += o[b];
       } else if constexpr (OUT == XYOut::SetInterior) {
-        if (interior) outp[gi] = o[b];
+        if (interior) {
+          outp[gi] = o[b];
+          if (zero) zero[gi] = T(0);
+        }
       } else {
         outp[gi] = o[b];
       }
@@ -297,10 +301,12 @@ __global__ void prolong_z_kernel(T *__restrict__ tmp, const T *__restrict__ coar
   if (c == n_cells_c - 1) tmp[(N1f - 1) * P + idx] = MASK ? T(0) : v[K];
 }
 
-// z pass, restriction: tmp (N1f planes of P = N1c^2 entries) -> coarse.
+// z pass, restriction: tmp (N1f planes of P = N1c^2 entries) -> coarse.  zero
+// (may be null): a vector of the same layout whose interior is zeroed with it
+// (the V-cycle's next solution vector, without a fill of its own).
 template <int K, typename T, bool ADD>
 __global__ void restrict_z_kernel(T *__restrict__ coarse, const T *__restrict__ tmp, int N1c,
-                                  int N1f, int64_t c_sy, int64_t c_sz)
+                                  int N1f, int64_t c_sy, int64_t c_sz, T *__restrict__ zero)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
   const int64_t P = static_cast<int64_t>(N1c) * N1c;
@@ -320,11 +326,13 @@ __global__ void restrict_z_kernel(T *__restrict__ coarse, const T *__restrict__ 
   for (int b = 0; b < K; ++b) {
     const int gz = c * K + b;
     if (gz == 0 || gz >= N1c - 1) continue;
-    T &dst = coarse[gz * c_sz + gy * c_sy + gx];
-    if constexpr (ADD)
-      dst += o[b];
-    else
-      dst = o[b];
+    const int64_t at = gz * c_sz + gy * c_sy + gx;
+    if constexpr (ADD) {
+      coarse[at] += o[b];
+    } else {
+      coarse[at] = o[b];
+      if (zero) zero[at] = T(0);
+    }
   }
 }
 

@@ -210,3 +210,30 @@ def test_kappa_operator_tiles(cuda, oracle, k, n, dtype):
     torch.cuda.synchronize()
     assert relerr(y.cpu().numpy(), oracle.laplace_vmult(3, k, n, x, kappa=kap)) < TOL[dtype]
     P.close()
+
+
+@pytest.mark.parametrize("dim,k,n", [(2, 3, 16), (3, 3, 12), (3, 4, 8)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_vcycle_after_calls_that_leave_its_vectors_dirty(cuda, dim, k, n, precision):
+    """A V-cycle starts from zero whatever ran before it on the handle's work
+    vectors: timed sweeps, tensor-core sweeps on caller vectors with nonzero
+    boundary entries, solves, FMG, other V-cycles."""
+    P, Q = tps.PoissonProblem(dim, k, n), tps.PoissonProblem(dim, k, n)
+    b = torch.tensor(np.random.default_rng(2).uniform(-1, 1, P.n_dofs()), device="cuda")
+    ref, out = P.new_vector(), P.new_vector()
+    tps.MultigridSolvers(Q).vmult(ref, b, precision=precision)
+    MG = tps.MultigridSolvers(P)
+    v = torch.rand(P.n_dofs(), device="cuda") + 1.0
+    dirty = [lambda: [P.time_smoother(lv, precision, 2) for lv in range(P.n_levels)],
+             lambda: MG.solve_cg(b, precision=precision),
+             lambda: MG.solve_fmg([torch.ones_like(P.new_vector(lv)) for lv in range(P.n_levels)], precision=precision),
+             lambda: MG.vmult(out, 2.0 * b, precision=precision, symmetric=True)]
+    if dim == 3:
+        dirty.append(lambda: tps.PatchSmoother(P, tensor_cores=True).step(v, v.clone()))
+    for f in dirty:
+        f()
+        MG.vmult(out, b, precision=precision)
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+    P.close()
+    Q.close()
