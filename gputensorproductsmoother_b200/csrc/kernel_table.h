@@ -58,6 +58,11 @@ struct KernelTable {
   cudaError_t (*smoother[2][2])(const LevelGeomH &, const VecLayout &, void *x, const void *b,
                                 int colour, double omega, int zero_x, int variant,
                                 const SmootherMaps *maps, int *err, cudaStream_t);
+  // the whole coloured sweep as one launch of one cluster; sweep_pays: whether
+  // that is the faster form on a level of n cells
+  cudaError_t (*sweep[2][2])(const LevelGeomH &, const VecLayout &, void *x, const void *b, int reverse,
+                             double omega, int zero_x, cudaStream_t);
+  bool (*sweep_pays)(int dim, int dtype, int n);
   // TMA descriptors of the 3D smoother for vectors x, b with layout l ([dtype])
   cudaError_t (*encode_maps[2])(const VecLayout &l, void *x, const void *b, SmootherMaps *out);
   // fine += P coarse (interior fine DoFs); geometry of the COARSE level

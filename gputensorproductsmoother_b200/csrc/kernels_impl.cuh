@@ -20,6 +20,7 @@
 #include "smoother3d_tc.cuh"
 #include "smoother3d_warp.cuh"
 #include "smoother_variants.cuh"
+#include "sweep_cluster.cuh"
 #include "transfer.cuh"
 
 namespace tps {
@@ -120,6 +121,8 @@ cudaError_t set_attributes()
     TPS_SET((smoother3d_warp_kernel<K, T, wp3_warps<K, T>()>), (Wp3<K, T, wp3_warps<K, T>()>::BYTES));
   if constexpr (sizeof(T) == 4 && pp3_enabled<K>())
     TPS_SET((smoother3d_pair_kernel<K, pp3_warps<K>()>), (Pp3<K, pp3_warps<K>()>::BYTES));
+  TPS_SET((sweep2d_kernel<K, T>), (Sw2<K, T>::BYTES));
+  TPS_SET((sweep3d_kernel<K, T>), (Sw3<K, T>::BYTES));
   TPS_SET((laplace_kernel<2, K, T, OpMode::Vmult>), (laplace_smem<2, T>()));
   TPS_SET((laplace_kernel<2, K, T, OpMode::Residual>), (laplace_smem<2, T>()));
   TPS_SET((laplace3d_march_kernel<K, T, OpMode::Vmult, false>), (sizeof(T) * OpMarch<K, T>::ELEMS));
@@ -401,6 +404,57 @@ cudaError_t smoother(const LevelGeomH &g, const VecLayout &l, void *x, const voi
       smoother3d_launch<T, sm3_variant_ppb<K, T, 2>()>(a, maps, x, b, scale, fd, err, s);
     else
       smoother3d_launch<T, sm3_variant_ppb<K, T, 0>()>(a, maps, x, b, scale, fd, err, s);
+  }
+  return cudaGetLastError();
+}
+
+// Whether a level's sweep runs as one launch of one cluster (sweep_cluster.cuh).
+// Measured, us per sweep, one launch / a launch per colour:
+//   2D, one CTA (at most 7 warps of patches in the largest colour): FP64 Q1 16^2
+//   5.0 / 13.3, Q2 8^2 6.9 / 9.6, Q2 16^2 8.4 / 9.4, Q5 8^2 11.0 / 15.9, Q7 4^2 14.1 /
+//   18.6; FP32 Q2 16^2 7.4 / 9.8, Q4 8^2 7.8 / 9.7; but with 8 warps Q7 8^2 FP64
+//   19.3 / 18.9, and with the barrier of several CTAs Q3 32^2 15.7 / 10.4;
+//   3D, a patch per CTA up to 8 CTAs: FP32 Q4 4^3 18.2 / 29.9, Q4 8^3 22.5 / 31.1,
+//   Q1 8^3 13.5 / 27.4, Q7 4^3 47.6 / 61.4; FP64 Q3 8^3 25.7 / 27.0, Q4 4^3 26.3 /
+//   30.8; but Q4 8^3 FP64 35.7 / 32.6, Q5 8^3 FP32 42.9 / 38.5.
+// Two cells per direction have one patch and one launch as it is.
+bool sweep_pays(int dim, int dtype, int n)
+{
+  if (n < 3) return false;
+  const int c = n / 2;  // patches per direction of the largest colour
+  if (dim == 2) return ceil_div(int64_t(c) * c, 32 / (2 * K - 1)) <= 7;
+  const int count = c * c * c;
+  if (n < 10 && count <= 8) return !(K == 5 && dtype == 0);
+  return n < 10 && count <= 64 && (K <= 3 || (K == 4 && dtype == 1));
+}
+
+template <int DIM, typename T>
+cudaError_t sweep(const LevelGeomH &g, const VecLayout &l, void *x, const void *b, int reverse, double omega,
+                  int zero_x, cudaStream_t s)
+{
+  int nx, ny, nz, count;
+  colour_lattice(DIM, g.n, 0, nx, ny, nz, count);  // the largest colour
+  if (count == 0) return cudaSuccess;
+  const double sc = stiffness_scale(DIM, g.h);
+  SweepArgs a;
+  a.n = g.n;
+  a.reverse = reverse;
+  a.zero_x = zero_x;
+  a.sy = l.sy;
+  a.sz = l.sz;
+  magic_div(static_cast<uint32_t>(nx), a.m0, a.s0);
+  magic_div(static_cast<uint32_t>(g.n > 2 ? (g.n - 1) / 2 : 1), a.m1, a.s1);
+  if constexpr (DIM == 2) {
+    const int need = static_cast<int>(ceil_div(count, Sm2<K, T>::P));
+    const int warps = need < Sw2<K, T>::WARPS ? need : Sw2<K, T>::WARPS;
+    (void)launch_cluster(sweep2d_kernel<K, T>, 1, 32 * warps, Sm2<K, T>::WARP_BYTES * warps, s,
+                         static_cast<T *>(x), static_cast<const T *>(b), a, static_cast<T>(sc),
+                         static_cast<T>(omega / sc));
+  } else {
+    // a patch per CTA, up to the portable cluster of 8; a CTA then takes more
+    const int ctas = count > 4 ? 8 : count > 2 ? 4 : count;
+    (void)launch_cluster(sweep3d_kernel<K, T>, ctas, Sw3<K, T>::NT, Sw3<K, T>::BYTES, s, static_cast<T *>(x),
+                         static_cast<const T *>(b), a, static_cast<T>(sc), static_cast<T>(omega / sc));
   }
   return cudaGetLastError();
 }
@@ -843,6 +897,9 @@ const KernelTable TPS_CAT(kernel_table_k, TPS_DEGREE) = {
      {&deg_impl::laplace<3, double>, &deg_impl::laplace<3, float>}},
     {{&deg_impl::smoother<2, double>, &deg_impl::smoother<2, float>},
      {&deg_impl::smoother<3, double>, &deg_impl::smoother<3, float>}},
+    {{&deg_impl::sweep<2, double>, &deg_impl::sweep<2, float>},
+     {&deg_impl::sweep<3, double>, &deg_impl::sweep<3, float>}},
+    &deg_impl::sweep_pays,
     {&deg_impl::encode_maps<double>, &deg_impl::encode_maps<float>},
     {{&deg_impl::prolong<2, double>, &deg_impl::prolong<2, float>},
      {&deg_impl::prolong<3, double>, &deg_impl::prolong<3, float>}},

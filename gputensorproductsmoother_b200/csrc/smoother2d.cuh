@@ -68,36 +68,45 @@ struct Sm2Args {
   uint32_t mx, sx;   // n / nx_c == (n * mx) >> sx
 };
 
+// What a lane keeps from patch to patch: its place in the warp's patches, its
+// rows of M and L, its 1 / lambda sums, and its patch's buffers.
 template <int K, typename T>
-__global__ void __launch_bounds__(32 * Sm2<K, T>::MAX_WARPS)
-    smoother2d_kernel(T *__restrict__ x, const T *__restrict__ b, const Sm2Args a, T scale, T fd_scale)
-{
+struct Sm2Lane {
   using S = Sm2<K, T>;
   using Q = Quad<T>;
-  constexpr int N1 = S::N1, M = S::M, P = S::P;
-  const DegreeTables<K, T> &tb = c_tables<K, T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // lanes past the last patch repeat lane 0 of patch 0 and write nothing
-  const bool own = lane < P * M;
-  const int p = own ? lane / M : 0, l = own ? lane - p * M : 0;
-  Q *ring = reinterpret_cast<Q *>(smem_raw + warp * S::WARP_BYTES) + p * S::PATCH_QUADS;
-  Q *line = ring + N1;
-  T *tr = reinterpret_cast<T *>(line + M);
-  // this lane's rows of M and L, and its 1 / lambda sums
+  static constexpr int N1 = S::N1, M = S::M, P = S::P;
+  bool own;  // lanes past the last patch repeat lane 0 of patch 0 and write nothing
+  int p, l;
+  Q *ring, *line;
+  T *tr;
   T rm[N1], rl[N1], rlam[M];
-#pragma unroll
-  for (int j = 0; j < N1; ++j) {
-    rm[j] = g_prows2<K, T>[j * M + l];
-    rl[j] = g_prows2<K, T>[(N1 + j) * M + l];
-  }
-#pragma unroll
-  for (int j = 0; j < M; ++j) rlam[j] = fd_scale * g_rlam2<K, T>[j * M + l];  // symmetric
-  const int sy = static_cast<int>(a.sy);  // a patch spans less than 2^31 entries
 
-  griddep_wait();  // programmatic launch: the previous kernel's writes are visible
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int w = blockIdx.x * (blockDim.x >> 5) + warp; w * P < a.count; w += nw) {
+  __device__ __forceinline__ Sm2Lane(unsigned char *warp_smem, T fd_scale)
+  {
+    const int lane = threadIdx.x & 31;
+    own = lane < P * M;
+    p = own ? lane / M : 0;
+    l = own ? lane - p * M : 0;
+    ring = reinterpret_cast<Q *>(warp_smem) + p * S::PATCH_QUADS;
+    line = ring + N1;
+    tr = reinterpret_cast<T *>(line + M);
+#pragma unroll
+    for (int j = 0; j < N1; ++j) {
+      rm[j] = g_prows2<K, T>[j * M + l];
+      rl[j] = g_prows2<K, T>[(N1 + j) * M + l];
+    }
+#pragma unroll
+    for (int j = 0; j < M; ++j) rlam[j] = fd_scale * g_rlam2<K, T>[j * M + l];  // symmetric
+  }
+
+  // One warp-load of patches (the w-th P patches of the colour).  COHERENT: x
+  // was written by other SMs earlier in this kernel, so it is read from L2.
+  template <bool COHERENT>
+  __device__ __forceinline__ void solve(T *x, const T *__restrict__ b, const Sm2Args &a, T scale, int w)
+  {
+    const DegreeTables<K, T> &tb = c_tables<K, T>;
+    const int sy = static_cast<int>(a.sy);  // a patch spans less than 2^31 entries
+    auto ld = [](const T *q) { return COHERENT ? __ldcg(q) : *q; };
     const int j0 = w * P + p;
     const bool valid = own && j0 < a.count;
     const int jp = valid ? j0 : w * P;
@@ -115,10 +124,10 @@ __global__ void __launch_bounds__(32 * Sm2<K, T>::MAX_WARPS)
       if (j < N1) {
         const bool corner = j == 0 || j == N1 - 1;
         Q q;
-        q.v[0] = xb[j];
-        q.v[1] = xb[j + (N1 - 1) * a.sy];
-        q.v[2] = corner ? T(0) : xb[j * a.sy];
-        q.v[3] = corner ? T(0) : xb[j * a.sy + N1 - 1];
+        q.v[0] = ld(xb + j);
+        q.v[1] = ld(xb + j + (N1 - 1) * a.sy);
+        q.v[2] = corner ? T(0) : ld(xb + j * a.sy);
+        q.v[3] = corner ? T(0) : ld(xb + j * a.sy + N1 - 1);
         if (own) ring[j] = q;
       }
     }
@@ -188,6 +197,19 @@ __global__ void __launch_bounds__(32 * Sm2<K, T>::MAX_WARPS)
     }
     __syncwarp();  // the ring and transposition buffers are read before the next patch
   }
+};
+
+template <int K, typename T>
+__global__ void __launch_bounds__(32 * Sm2<K, T>::MAX_WARPS)
+    smoother2d_kernel(T *x, const T *__restrict__ b, const Sm2Args a, T scale, T fd_scale)
+{
+  using S = Sm2<K, T>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  Sm2Lane<K, T> lane(smem_raw + warp * S::WARP_BYTES, fd_scale);
+  griddep_wait();  // programmatic launch: the previous kernel's writes are visible
+  for (int w = blockIdx.x * warps + warp; w * S::P < a.count; w += gridDim.x * warps)
+    lane.template solve<false>(x, b, a, scale, w);
 }
 
 }  // namespace tps

@@ -197,6 +197,7 @@ struct tps_handle {
   std::vector<int> coarse_coord;        // (x, y, z) of each interior coarse DoF
   VcycleVectors vc[2];  // [0] FP64, [1] FP32
   std::vector<int> sm_variant[2];  // per level: 3D smoother patches-per-batch variant (autotuned)
+  std::vector<char> sm_explicit[2];  // per level: chosen by tps_set_smoother_variant
   std::vector<int> op_layers[2];   // per level: 3D operator cell layers per CTA (autotuned; 0 default)
   DevBuf dot_part;                 // 3D: per-CTA p.q partial sums of the fused CG operator
   int dot_cap = 0;                 // their capacity
@@ -462,6 +463,11 @@ void smoother_sweep(tps_handle *h, int level, int p, const VecLayout &lay, void 
   const int variant = level < static_cast<int>(h->sm_variant[p].size()) ? h->sm_variant[p][level]
                                                                         : default_variant(h, level, p);
   if (!h->err_flag.p) h->err_flag.alloc(sizeof(int));
+  const bool chosen = level < static_cast<int>(h->sm_explicit[p].size()) && h->sm_explicit[p][level];
+  if (!use_tc && !h->has_kappa && !chosen && h->kt->sweep_pays(h->dim, p, h->lv[level].n)) {
+    TPS_CUDA(h->kt->sweep[h->dim - 2][p](h->lv[level], lay, x, b, reverse ? 1 : 0, h->omega, x_zero ? 1 : 0, s));
+    return;
+  }
   const int nc = 1 << h->dim;
   for (int i = 0; i < nc; ++i) {
     const int c = reverse ? nc - 1 - i : i;
@@ -976,6 +982,7 @@ void autotune_levels(tps_handle *h, int p, cudaStream_t s)
   ensure_krylov(h);
   h->sm_variant[p].assign(h->n_levels, 0);
   h->op_layers[p].assign(h->n_levels, 0);
+  h->sm_explicit[p].assign(h->n_levels, 0);
   if (h->dim != 3 || h->has_kappa) return;
   for (int l = 0; l < h->n_levels; ++l) {
     float best_op = 1e30f;
@@ -993,6 +1000,10 @@ void autotune_levels(tps_handle *h, int p, cudaStream_t s)
     h->op_layers[p][l] = bz;
   }
   for (int l = 0; l < h->n_levels; ++l) {
+    if (h->kt->sweep_pays(3, p, h->lv[l].n)) {  // one launch per sweep, whatever the variant
+      h->sm_variant[p][l] = default_variant(h, l, p);
+      continue;
+    }
     float best = 1e30f;
     int bv = 0;
     for (int v = 0; v < kSmootherVariants; ++v) {
@@ -1671,6 +1682,8 @@ int tps_set_smoother_variant(tps_handle *h, int dtype, int level, int variant)
     if (variant < 0 || variant >= kSmootherVariants) throw ApiError(TPS_ERR_INVALID, "variant out of range");
     if (static_cast<int>(h->sm_variant[p].size()) != h->n_levels) h->sm_variant[p].assign(h->n_levels, 0);
     h->sm_variant[p][level] = variant;
+    if (static_cast<int>(h->sm_explicit[p].size()) != h->n_levels) h->sm_explicit[p].assign(h->n_levels, 0);
+    h->sm_explicit[p][level] = 1;
     if (h->graph) {  // later solves re-capture with the chosen kernel
       cudaGraphExecDestroy(h->graph);
       h->graph = nullptr;

@@ -317,7 +317,10 @@ int tps_set_smoother_variant(tps_handle *h, int dtype, int level, int variant);
  *   - one warp per patch at degree 4, and at degree 3 where a colour holds
  *     at least 4096 patches;
  *   - otherwise quarter CTA batches at degrees 2 and 3, and the default batch
- *     at other degrees. */
+ *     at other degrees.
+ * On the smallest levels (at most 8 patches per colour, 64 at degrees up to 3
+ * and at degree 4 in FP32) a sweep is one launch of its own kernel, with the same
+ * results, unless tps_set_smoother_variant chose a variant for the level. */
 int tps_get_smoother_variant(tps_handle *h, int dtype, int level, int *variant);
 
 /* ---- batched solves (no reference counterpart) ----------------------------

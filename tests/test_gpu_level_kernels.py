@@ -237,3 +237,29 @@ def test_vcycle_after_calls_that_leave_its_vectors_dirty(cuda, dim, k, n, precis
         assert torch.equal(out, ref)
     P.close()
     Q.close()
+
+
+# levels whose sweep is one launch, and the first ones past its rule, at every
+# degree: the oracle's sweep, and bit-identical to the per-colour kernels (an
+# explicitly chosen variant in 3D)
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_single_launch_sweeps(cuda, oracle, dim, k, dtype):
+    for n in (3, 4, 5, 6, 8, 9, 10, 16):
+        if (tps.split_cells(n)[0] * k - 1) ** dim > 1400 or (dim == 3 and n * k > 36):
+            continue
+        sweep_matches(oracle, dim, k, n, dtype, seed=n, relaxation=0.95)
+        if dim == 3:
+            P = tps.PoissonProblem(dim, k, n)
+            S = tps.PatchSmoother(P)
+            b = torch.rand(P.n_dofs(), device="cuda", dtype=dtype)
+            x, y = torch.rand_like(b), None
+            y = x.clone()
+            S.step(x, b)
+            prec = "fp64" if dtype == torch.float64 else "fp32"
+            P.set_smoother_variant(0, prec)
+            S.step(y, b)
+            torch.cuda.synchronize()
+            assert torch.equal(x, y)
+            P.close()
