@@ -342,6 +342,54 @@ __global__ void cg_update_p_kernel(double *p, const void *z, int z_kind, PadMap 
     p[i] = load_kind(z, z_kind, pad_index(i, pm)) + beta * p[i];
 }
 
+// Every CTA sums the previous step's partial sums itself (the same 4.7 KB from
+// L2, in the order of reduce_kernel), so that a step is one launch and no scalar
+// goes to the host: with a dot, a reduction, a copy, a wait and an axpy per
+// vector the 5 iterations of a 3D Q3 24^3 solve spent 0.4 of 1.7 ms on them.
+__global__ void __launch_bounds__(kRedThreads)
+    mgs_step_kernel(double *__restrict__ w, const double *__restrict__ v_prev, const double *__restrict__ v_next,
+                    const double *__restrict__ in, double *__restrict__ h, double *__restrict__ out, int64_t n)
+{
+  griddep_wait();  // programmatic launch: the previous kernel's writes are visible
+  __shared__ double sh[32];
+  __shared__ double hv;
+  double a = 0.0;
+  if (in) {
+    double t = 0.0;
+    for (int i = threadIdx.x; i < kRedBlocks; i += kRedThreads) t += in[i];
+    t = block_sum<kRedThreads>(t, sh);
+    if (threadIdx.x == 0) {
+      hv = t;
+      if (blockIdx.x == 0) *h = t;
+    }
+    __syncthreads();
+    a = -hv;
+  }
+  double s = 0.0;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    double wi = w[i];
+    if (in) {
+      wi += a * v_prev[i];
+      w[i] = wi;
+    }
+    s += wi * (v_next ? v_next[i] : wi);
+  }
+  s = block_sum<kRedThreads>(s, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
+__global__ void __launch_bounds__(kRedThreads) mgs_finish_kernel(const double *in, const double *h, int n_h, double *dst)
+{
+  griddep_wait();  // programmatic launch: the previous kernel's writes are visible
+  __shared__ double sh[32];
+  double t = 0.0;
+  for (int i = threadIdx.x; i < kRedBlocks; i += kRedThreads) t += in[i];
+  t = block_sum<kRedThreads>(t, sh);
+  if (threadIdx.x == 0) dst[n_h] = t;
+  if (static_cast<int>(threadIdx.x) < n_h) dst[threadIdx.x] = h[threadIdx.x];
+}
+
 __global__ void axpy_kernel(double *y, double a, const double *x, int64_t n)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
@@ -558,6 +606,17 @@ cudaError_t launch_scale_f64(double *y, double a, int64_t n, cudaStream_t s)
 cudaError_t launch_sub_f64(double *dst, const double *a, const double *b, int64_t n, cudaStream_t s)
 {
   TPS_LAUNCH((sub_kernel), stream_grid(n, 256), 256, 0, s, dst, a, b, n);
+  return cudaGetLastError();
+}
+cudaError_t launch_mgs_step(double *w, const double *v_prev, const double *v_next, const double *in, double *h,
+                            double *out, int64_t n, cudaStream_t s)
+{
+  TPS_LAUNCH((mgs_step_kernel), kRedBlocks, kRedThreads, 0, s, w, v_prev, v_next, in, h, out, n);
+  return cudaGetLastError();
+}
+cudaError_t launch_mgs_finish(const double *in, const double *h, int n_h, double *dst, cudaStream_t s)
+{
+  TPS_LAUNCH((mgs_finish_kernel), 1, kRedThreads, 0, s, in, h, n_h, dst);
   return cudaGetLastError();
 }
 cudaError_t launch_to_vcycle(void *d, void *su, int d_kind, PadMap pm, const double *src, int64_t n,

@@ -103,6 +103,14 @@ cudaError_t launch_axpy_f64(double *y, double a, const double *x, int64_t n, cud
 cudaError_t launch_scale_f64(double *y, double a, int64_t n, cudaStream_t s);
 cudaError_t launch_sub_f64(double *dst, const double *a, const double *b, int64_t n,
                            cudaStream_t s);  // dst = a - b
+// One modified Gram-Schmidt step, with its scalars kept on the device: the
+// partial sums `in` (null at the first step) give h = <w, v_prev>, stored in *h;
+// w -= h v_prev; the partial sums of <w, v_next> (v_next null: <w, w>) go to
+// `out`.  in and out are two arrays of kRedBlocks entries.
+cudaError_t launch_mgs_step(double *w, const double *v_prev, const double *v_next, const double *in, double *h,
+                            double *out, int64_t n, cudaStream_t s);
+// dst[0 .. n_h - 1] = h, dst[n_h] = the sum of the partial sums (dst may be host-mapped)
+cudaError_t launch_mgs_finish(const double *in, const double *h, int n_h, double *dst, cudaStream_t s);
 // V-cycle input from an FP64 vector and FP64 output from the V-cycle result
 cudaError_t launch_to_vcycle(void *d, void *su, int d_kind, PadMap pm, const double *src, int64_t n,
                              cudaStream_t s);

@@ -1210,7 +1210,8 @@ int solve_gmres(tps_handle *h, const tps_solve_opts &o, const double *b, double 
   vcycle_vectors(h, vprec_index(o.precision));
   const LevelGeomH &g = h->fine();
   const int64_t N = g.N;
-  const int basis = 28;  // max_n_tmp_vectors - 2 with deal.II's default of 30
+  constexpr int basis = 28;  // max_n_tmp_vectors - 2 with deal.II's default of 30
+  static_assert(sizeof(double) * (basis + 1) <= Mailbox::kBytes, "a basis' coefficients and a norm fit the mailbox");
   const int nvec = std::min(basis, std::max(o.max_iter, 1)) + 1;
   while (static_cast<int>(h->gmres_v.size()) < nvec) {
     std::unique_ptr<DevBuf> v(new DevBuf);
@@ -1253,11 +1254,22 @@ int solve_gmres(tps_handle *h, const tps_solve_opts &o, const double *b, double 
       fine_vmult64(h, pv, Vp(inner), s);
       apply_vcycle64(h, o.precision, false, Vp(inner + 1), pv, s);
       dimk = inner + 1;
-      for (int i = 0; i < dimk; ++i) {
-        hv[i] = dev_dot(h, Vp(inner + 1), Vp(i), s);
-        TPS_CUDA(launch_axpy_f64(Vp(inner + 1), -hv[i], Vp(i), N, s));
-      }
-      const double sn = std::sqrt(dev_dot(h, Vp(inner + 1), Vp(inner + 1), s));
+      // orthogonalise against v_0 .. v_inner, the coefficients staying on the
+      // device until the norm of what is left comes with them
+      double *part = h->partial.as<double>(), *hd = part + 2 * kRedBlocks;
+      for (int i = 0; i <= dimk; ++i)
+        TPS_CUDA(launch_mgs_step(Vp(inner + 1), i > 0 ? Vp(i - 1) : nullptr, i < dimk ? Vp(i) : nullptr,
+                                 i > 0 ? part + ((i - 1) & 1) * kRedBlocks : nullptr, i > 0 ? hd + i - 1 : nullptr,
+                                 part + (i & 1) * kRedBlocks, N, s));
+      h->mbox.ensure();
+      void *mail = nullptr;
+      TPS_CUDA(cudaHostGetDevicePointer(&mail, h->mbox.host, 0));
+      TPS_CUDA(launch_mgs_finish(part + (dimk & 1) * kRedBlocks, hd, dimk, static_cast<double *>(mail), s));
+      TPS_CUDA(cudaStreamSynchronize(s));
+      std::memcpy(hv.data(), h->mbox.host, sizeof(double) * dimk);
+      double nn = 0.0;
+      std::memcpy(&nn, static_cast<const double *>(h->mbox.host) + dimk, sizeof(double));
+      const double sn = std::sqrt(nn);
       hv[inner + 1] = sn;
       if (sn != 0.0) TPS_CUDA(launch_scale_f64(Vp(inner + 1), 1.0 / sn, N, s));
       for (int i = 0; i < inner; ++i) {

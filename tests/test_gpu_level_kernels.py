@@ -263,3 +263,34 @@ def test_single_launch_sweeps(cuda, oracle, dim, k, dtype):
             torch.cuda.synchronize()
             assert torch.equal(x, y)
             P.close()
+
+
+# one iteration, restarts after a full basis (28 vectors), vectors shorter and
+# longer than the reductions' grid; the coefficients come from the device.  The
+# residual that the recurrence reports is |V(b - A x)| / |V b| in exact
+# arithmetic; rounding separates the two by about 2^-53 |V b| times the
+# operator's condition number (at most 1e6 here), so they are compared above
+# 1e-9 and both have to be below it otherwise.
+@pytest.mark.parametrize("dim,k,n,max_iter,reduce", [(2, 1, 4, 20, 1e-9), (2, 2, 256, 2, 1e-30), (2, 2, 256, 20, 1e-9),
+                                                      (3, 2, 16, 40, 1e-30), (3, 3, 24, 1, 1e-30), (3, 3, 24, 3, 1e-30)])
+def test_gmres_residual_is_the_reported_one(cuda, dim, k, n, max_iter, reduce):
+    P = tps.PoissonProblem(dim, k, n)
+    MG = tps.MultigridSolvers(P)
+    b = np.random.default_rng(8).uniform(-1, 1, (n * k + 1,) * dim)
+    for ax in range(dim):
+        np.moveaxis(b, ax, 0)[[0, -1]] = 0.0
+    b = torch.tensor(b.ravel(), device="cuda")
+    x, rep = MG.solve_gmres(b, precision="fp64", max_iter=max_iter, reduce=reduce)
+    r, z, z0 = P.new_vector(), P.new_vector(), P.new_vector()
+    tps.LaplaceOperator(P).vmult(r, x)
+    MG.vmult(z, b - r, precision="fp64")
+    MG.vmult(z0, b, precision="fp64")
+    torch.cuda.synchronize()
+    true = (z.norm() / z0.norm()).item()
+    # (an absolute tolerance of 1e-16 can end the long run early)
+    assert 1 <= rep.iterations <= max_iter and (rep.converged or reduce < 1e-20)
+    if rep.final_residual > 1e-9:
+        assert abs(true - rep.final_residual) < 1e-3 * rep.final_residual, (true, rep.final_residual)
+    else:
+        assert true < 1e-9, (true, rep.final_residual)
+    P.close()
