@@ -142,6 +142,8 @@ cudaError_t set_attributes()
                              cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
   }
+  TPS_SET((prolong3d_kernel<K, T, true>), (Prol3<K, T>::BYTES));
+  if constexpr (sizeof(T) == 8) TPS_SET((prolong3d_kernel<K, T, false>), (Prol3<K, T>::BYTES));
   TPS_SET((restrict_xy_kernel<K, T, XYOut::AddInterior>), (restrict_smem<T>()));
   TPS_SET((restrict_xy_kernel<K, T, XYOut::SetInterior>), (restrict_smem<T>()));
   TPS_SET((restrict_xy_kernel<K, T, XYOut::SetAll>), (restrict_smem<T>()));
@@ -622,21 +624,17 @@ template <int DIM, typename T, bool MASK>
 cudaError_t prolong_impl(const LevelGeomH &gc, const VecLayout &lc, const VecLayout &lf, void *fine,
                          const void *coarse, void *tmp, cudaStream_t s)
 {
-  constexpr int C = ProlTile<K, T>::C;
   const int N1c = gc.N1, N1f = 2 * gc.n * K + 1;
-  const unsigned gxy = ceil_div(gc.n, C);
   if constexpr (DIM == 2) {
+    const unsigned gxy = ceil_div(gc.n, ProlTile<K, T>::C);
+    (void)tmp;
     TPS_LAUNCH((prolong_xy_kernel<K, T, XYOut::AddInterior>), dim3(gxy, gxy, 1), XYTile<K>::NT, 0, s,
         static_cast<T *>(fine), static_cast<const T *>(coarse), N1c, N1f, lc.sy, 0, lf.sy, 0, 0, MASK ? 1 : 0);
   } else {
-    const int64_t P = static_cast<int64_t>(N1c) * N1c;
-    TPS_LAUNCH((prolong_z_kernel<K, T, MASK>), dim3(ceil_div(P, 256), gc.n), 256, 0, s,
-        static_cast<T *>(tmp), static_cast<const T *>(coarse), N1c, N1f, gc.n, lc.sy, lc.sz);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    // fine interior planes 1..N1f-2 from tmp planes 1..N1f-2
-    TPS_LAUNCH((prolong_xy_kernel<K, T, XYOut::AddInterior>), dim3(gxy, gxy, N1f - 2), XYTile<K>::NT, 0, s,
-        static_cast<T *>(fine), static_cast<const T *>(tmp), N1c, N1f, N1c, P, lf.sy, lf.sz, 1, MASK ? 1 : 0);
+    using S = Prol3<K, T>;
+    (void)tmp;
+    TPS_LAUNCH((prolong3d_kernel<K, T, MASK>), dim3(ceil_div(gc.n, S::TX), ceil_div(gc.n, S::TY), gc.n), S::NT,
+        S::BYTES, s, static_cast<T *>(fine), static_cast<const T *>(coarse), N1c, N1f, lc.sy, lc.sz, lf.sy, lf.sz);
   }
   return cudaGetLastError();
 }

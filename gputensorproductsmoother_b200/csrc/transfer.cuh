@@ -275,30 +275,107 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
 }
 
 // ---------------------------------------------------------------------------
-// z pass, prolongation: coarse (N1c planes of P entries) -> tmp (N1f planes of
-// P entries), P = N1c^2.  Input entries on the coarse boundary read as zero
-// (MASK) or as they are (the FMG prolongation of the solution).
-template <int K, typename T, bool MASK = true>
-__global__ void prolong_z_kernel(T *__restrict__ tmp, const T *__restrict__ coarse, int N1c,
-                                 int N1f, int n_cells_c, int64_t c_sy, int64_t c_sz)
+// 3D prolongation in one pass: fine interior += P coarse for the fine nodes of a
+// tile of TX x TY coarse cells in one cell layer.  The tile's coarse box is
+// contracted in z, x and y through shared memory (the order of the passes over
+// whole levels that it replaces, so the same rounding), while the current fine
+// values of the thread's (z, x) columns are already on their way.  Coarse
+// boundary entries read as zero (MASK) or as they are (the FMG prolongation of
+// the solution).
+//
+// What bounds it: HBM and the latency of three short stages; the coarse box is
+// read about 1.5 times (L2), the intermediate fine-z level (a quarter of the
+// fine one, written and read) is gone, and so is one launch.  Measured, us per
+// prolongate-and-add, two passes / now: Q4 64^3 FP64 82 / 72, FP32 53 / 40; Q7 32^3
+// FP64 129 / 39, FP32 94 / 27; Q5 32^3 FP64 45 / 17; Q2 96^3 FP64 41 / 21; Q4 8^3
+// 18 / 14.
+template <int K, typename T>
+struct Prol3 {
+  static constexpr int TX = K == 1 ? 16 : K == 2 ? 8 : K == 3 ? 5 : K == 4 ? 4 : K == 5 ? 3 : 2;
+  static constexpr int TY = K == 1 ? 8 : K == 2 ? 4 : K <= 4 ? 2 : 1;
+  static constexpr int NT = 256;
+  static constexpr int CX = TX * K + 1, CY = TY * K + 1, F = 2 * K, WX = F * TX;
+  static constexpr int CB = (K + 1) * CY * CX, ZB = F * CY * CX, XB = F * CY * WX;
+  static constexpr int YTASKS = F * TY * WX, YPT = (YTASKS + NT - 1) / NT;
+  // the x-contracted lines take the place of the coarse box
+  static constexpr int R0 = CB > XB ? CB : XB;
+  static constexpr size_t BYTES = sizeof(T) * (R0 + ZB);
+};
+
+template <int K, typename T, bool MASK>
+__global__ void __launch_bounds__(Prol3<K, T>::NT)
+    prolong3d_kernel(T *__restrict__ fine, const T *__restrict__ coarse, int N1c, int N1f, int64_t c_sy, int64_t c_sz,
+                     int64_t f_sy, int64_t f_sz)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
-  const int64_t P = static_cast<int64_t>(N1c) * N1c;
-  const int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int c = blockIdx.y;  // coarse cell along z
-  if (idx >= P) return;
-  const int gy = static_cast<int>(idx) / N1c, gx = static_cast<int>(idx) - gy * N1c;  // idx < N1c^2 < 2^31
-  const bool bxy = gx == 0 || gx == N1c - 1 || gy == 0 || gy == N1c - 1;
-  T v[K + 1], o[2 * K];
-#pragma unroll
-  for (int b = 0; b <= K; ++b) {
-    const int gz = c * K + b;
-    v[b] = (MASK && (bxy || gz == 0 || gz == N1c - 1)) ? T(0) : __ldg(&coarse[gz * c_sz + gy * c_sy + gx]);
+  using S = Prol3<K, T>;
+  constexpr int NT = S::NT, F = S::F, CX = S::CX, CY = S::CY, WX = S::WX;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  T *sC = reinterpret_cast<T *>(smem_raw), *sX = sC, *sZ = sC + S::R0;
+  const int gx0 = blockIdx.x * S::TX * K, gy0 = blockIdx.y * S::TY * K, gz0 = blockIdx.z * K;
+  const uint32_t s_c = smem_u32(sC);
+  for (int e = threadIdx.x; e < S::CB; e += NT) {
+    const int r = e / CX, lx = e - r * CX, lz = r / CY, ly = r - lz * CY;
+    const int gx = gx0 + lx, gy = gy0 + ly, gz = gz0 + lz;
+    const bool in = gx < N1c && gy < N1c &&
+                    (!MASK || (gx > 0 && gx < N1c - 1 && gy > 0 && gy < N1c - 1 && gz > 0 && gz < N1c - 1));
+    cp_async_zfill_s<sizeof(T)>(s_c + static_cast<uint32_t>(sizeof(T) * e),
+                                in ? coarse + gx + gy * c_sy + gz * c_sz : coarse,
+                                in ? static_cast<uint32_t>(sizeof(T)) : 0u);
   }
-  prol_cell<K, T>(v, o);
+  cp_async_commit();
+  // y task: fine plane, coarse cell in y, fine column; its 2k current values
+  T cur[S::YPT][F];
 #pragma unroll
-  for (int f = 0; f < 2 * K; ++f) tmp[(2 * K * c + f) * P + idx] = o[f];
-  if (c == n_cells_c - 1) tmp[(N1f - 1) * P + idx] = MASK ? T(0) : v[K];
+  for (int u = 0; u < S::YPT; ++u) {
+    const int t = threadIdx.x + u * NT, r = t / WX, xx = t - r * WX, pz = r / S::TY, c = r - pz * S::TY;
+    const int gx = 2 * gx0 + xx, gz = 2 * gz0 + pz, gy1 = 2 * gy0 + c * F;
+    const bool col = t < S::YTASKS && gx > 0 && gx < N1f - 1 && gz > 0 && gz < N1f - 1;
+    const T *q = fine + gx + gz * f_sz + gy1 * f_sy;
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const int gy = gy1 + f;
+      cur[u][f] = col && gy > 0 && gy < N1f - 1 ? q[f * f_sy] : T(0);
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  for (int t = threadIdx.x; t < CX * CY; t += NT) {
+    T v[K + 1], o[F];
+#pragma unroll
+    for (int b = 0; b <= K; ++b) v[b] = sC[b * CX * CY + t];
+    prol_cell<K, T>(v, o);
+#pragma unroll
+    for (int f = 0; f < F; ++f) sZ[f * CX * CY + t] = o[f];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < F * CY * S::TX; t += NT) {
+    const int r = t / S::TX, c = t - r * S::TX;  // r: (fine plane, coarse row)
+    T v[K + 1], o[F];
+#pragma unroll
+    for (int b = 0; b <= K; ++b) v[b] = sZ[r * CX + c * K + b];
+    prol_cell<K, T>(v, o);
+#pragma unroll
+    for (int f = 0; f < F; ++f) sX[r * WX + c * F + f] = o[f];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < S::YPT; ++u) {
+    const int t = threadIdx.x + u * NT, r = t / WX, xx = t - r * WX, pz = r / S::TY, c = r - pz * S::TY;
+    const int gx = 2 * gx0 + xx, gz = 2 * gz0 + pz, gy1 = 2 * gy0 + c * F;
+    if (t < S::YTASKS && gx > 0 && gx < N1f - 1 && gz > 0 && gz < N1f - 1) {
+      T v[K + 1], o[F];
+#pragma unroll
+      for (int b = 0; b <= K; ++b) v[b] = sX[(pz * CY + c * K + b) * WX + xx];
+      prol_cell<K, T>(v, o);
+      T *q = fine + gx + gz * f_sz + gy1 * f_sy;
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const int gy = gy1 + f;
+        if (gy > 0 && gy < N1f - 1) q[f * f_sy] = cur[u][f] + o[f];
+      }
+    }
+  }
 }
 
 // z pass, restriction: tmp (N1f planes of P = N1c^2 entries) -> coarse.  zero

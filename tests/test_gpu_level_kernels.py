@@ -294,3 +294,21 @@ def test_gmres_residual_is_the_reported_one(cuda, dim, k, n, max_iter, reduce):
     else:
         assert true < 1e-9, (true, rep.final_residual)
     P.close()
+
+
+# tiles with remainders in x and y at every degree; adds to what is there, on
+# interior fine nodes only
+@pytest.mark.parametrize("k,n", [(1, 6), (1, 40), (2, 20), (3, 12), (4, 12), (5, 8), (6, 8), (7, 8)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_prolongation_tiles(cuda, oracle, k, n, dtype):
+    P = tps.PoissonProblem(3, k, n)
+    npdt = np.float64 if dtype == torch.float64 else np.float32
+    rng = np.random.default_rng(23)
+    L = P.n_levels - 1
+    c, f = rng.uniform(-1, 1, P.n_dofs(L - 1)).astype(npdt), rng.uniform(-1, 1, P.n_dofs()).astype(npdt)
+    ref = oracle.prolongate_add(3, k, n // 2, f, c)
+    got = torch.tensor(f, device="cuda")
+    tps.MGTransferCUDA(P).prolongate_and_add(L, got, torch.tensor(c, device="cuda"))
+    torch.cuda.synchronize()
+    assert relerr(got.cpu().numpy(), ref) < TOL[dtype]
+    P.close()
