@@ -199,7 +199,6 @@ cudaError_t launch_spd_inverse(double *a, double *tmp, int n, int *bad, cudaStre
 {
   cudaError_t e = cudaFuncSetAttribute(gauss_jordan_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(SweepSmem)));
-  if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   const unsigned t = static_cast<unsigned>((n + kTile - 1) / kTile);
   double *src = a, *dst = tmp;

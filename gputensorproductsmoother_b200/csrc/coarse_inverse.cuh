@@ -16,7 +16,7 @@ struct CoarseOperator {
 // a (ni x ni, ni interior DoFs lexicographic) = the interior operator
 cudaError_t launch_assemble_coarse(double *a, const CoarseOperator &q, int ni, cudaStream_t s);
 // a <- a^-1 for a symmetric positive definite a (n x n), tmp of the same size;
-// *bad (device) is set to 1 where a pivot is not positive, else to 0
+// *bad (device, 0 on entry) is set to 1 where a pivot is not positive
 cudaError_t launch_spd_inverse(double *a, double *tmp, int n, int *bad, cudaStream_t s);
 
 }  // namespace tps

@@ -100,10 +100,6 @@ struct IntC {
   static constexpr int value = V;
 };
 
-// 1 / (lambda_x + lambda_y + lambda_z) of the interior modes, z-major
-template <int K, typename T>
-__device__ T g_rlam3[(2 * K - 1) * (2 * K - 1) * (2 * K - 1)];
-
 // rows Y0+1 .. Y0+NY (y) and 1..k (z) of the cell product of one thread:
 // acc[z][y] = L_z M_y TA + M_z (L_y TA + M_y TB); ta, tb point at the cell's
 // outermost (z, y) entry of this x node, dz and dy step inward
@@ -303,7 +299,7 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
     for (int i = 0; i < M; ++i) v[i] = TA[i * PM + t];
     evec_apply<K, T, true>(v, q);
 #pragma unroll
-    for (int i = 0; i < M; ++i) q[i] *= fd_scale * g_rlam3<K, T>[i * PM + t];
+    for (int i = 0; i < M; ++i) q[i] *= fd_scale * g_lane_tables<K, T>.rlam3[i * PM + t];
     evec_apply<K, T, false>(q, v);
 #pragma unroll
     for (int i = 0; i < M; ++i) TB[i * PM + t] = v[i];

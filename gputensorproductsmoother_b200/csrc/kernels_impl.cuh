@@ -69,23 +69,20 @@ cudaError_t upload_one(const DegreeData &D)
   for (int r = 0; r < C; ++r)
     for (int q = 0; q < C; ++q)
       t.evec_p[r * C + q] = Pair<T>::make(t.evec[r * M + q], t.evec[r * M + C + 1 + q]);
-  std::vector<T> rlam(static_cast<size_t>(M) * M * M);
+  std::vector<LaneTables<K, T>> lane(1);  // too large for the stack at degree 7
+  LaneTables<K, T> &lt = lane[0];
   for (int z = 0; z < M; ++z)
     for (int y = 0; y < M; ++y)
       for (int x = 0; x < M; ++x)
-        rlam[(static_cast<size_t>(z) * M + y) * M + x] = static_cast<T>(1.0 / (D.eval[x] + D.eval[y] + D.eval[z]));
-  cudaError_t e = cudaMemcpyToSymbol(g_rlam3<K, T>, rlam.data(), sizeof(T) * rlam.size());
-  if (e != cudaSuccess) return e;
-  std::vector<T> rows(2 * N1 * M), rlam2(M * M);
+        lt.rlam3[(z * M + y) * M + x] = static_cast<T>(1.0 / (D.eval[x] + D.eval[y] + D.eval[z]));
+  for (int y = 0; y < M; ++y)
+    for (int x = 0; x < M; ++x) lt.rlam2[y * M + x] = static_cast<T>(1.0 / (D.eval[y] + D.eval[x]));
   for (int j = 0; j < N1; ++j)
     for (int r = 0; r < M; ++r) {
-      rows[j * M + r] = static_cast<T>(D.pmass[(r + 1) * N1 + j]);
-      rows[(N1 + j) * M + r] = static_cast<T>(D.plap[(r + 1) * N1 + j]);
+      lt.prows2[j * M + r] = static_cast<T>(D.pmass[(r + 1) * N1 + j]);
+      lt.prows2[(N1 + j) * M + r] = static_cast<T>(D.plap[(r + 1) * N1 + j]);
     }
-  for (int y = 0; y < M; ++y)
-    for (int x = 0; x < M; ++x) rlam2[y * M + x] = static_cast<T>(1.0 / (D.eval[y] + D.eval[x]));
-  e = cudaMemcpyToSymbol(g_prows2<K, T>, rows.data(), sizeof(T) * rows.size());
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_rlam2<K, T>, rlam2.data(), sizeof(T) * rlam2.size());
+  const cudaError_t e = cudaMemcpyToSymbol(g_lane_tables<K, T>, &lt, sizeof(lt));
   if (e != cudaSuccess) return e;
   return cudaMemcpyToSymbol(c_tables<K, T>, &t, sizeof(t));
 }

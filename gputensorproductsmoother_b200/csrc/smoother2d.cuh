@@ -54,13 +54,6 @@ struct Sm2 {
   static constexpr int MAX_WARPS = 4;
 };
 
-// rows 1..2k-1 of the patch mass and stiffness, entry-major: [matrix][j][row]
-template <int K, typename T>
-__device__ T g_prows2[2 * (2 * K + 1) * (2 * K - 1)];
-// 1 / (lambda_y + lambda_x), [y mode][x mode]
-template <int K, typename T>
-__device__ T g_rlam2[(2 * K - 1) * (2 * K - 1)];
-
 struct Sm2Args {
   int nx_c, count;   // patches of the colour per row, and in all
   int cx, cy;        // colour parities
@@ -92,11 +85,11 @@ struct Sm2Lane {
     tr = reinterpret_cast<T *>(line + M);
 #pragma unroll
     for (int j = 0; j < N1; ++j) {
-      rm[j] = g_prows2<K, T>[j * M + l];
-      rl[j] = g_prows2<K, T>[(N1 + j) * M + l];
+      rm[j] = g_lane_tables<K, T>.prows2[j * M + l];
+      rl[j] = g_lane_tables<K, T>.prows2[(N1 + j) * M + l];
     }
 #pragma unroll
-    for (int j = 0; j < M; ++j) rlam[j] = fd_scale * g_rlam2<K, T>[j * M + l];  // symmetric
+    for (int j = 0; j < M; ++j) rlam[j] = fd_scale * g_lane_tables<K, T>.rlam2[j * M + l];  // symmetric
   }
 
   // One warp-load of patches (the w-th P patches of the colour).  COHERENT: x

@@ -192,8 +192,8 @@ struct tps_handle {
   bool dense_coarse = false;
   int n_int_coarse = 0;
   DevBuf coarse_inv;                    // n_int^2, FP64
-  DevBuf coarse_work[2];                // its assembly and inversion
-  DevBuf coarse_tab;                    // reference-cell mass and stiffness, the inversion's flag
+  std::vector<double> coarse_inv_host;  // a small one, until the first V-cycle needs it on the device
+  DevBuf coarse_work;                   // reference-cell mass and stiffness, the inversion's flag, its two matrices
   std::vector<int> coarse_coord;        // (x, y, z) of each interior coarse DoF
   VcycleVectors vc[2];  // [0] FP64, [1] FP32
   std::vector<int> sm_variant[2];  // per level: 3D smoother patches-per-batch variant (autotuned)
@@ -292,36 +292,102 @@ int guarded(tps_handle *h, F &&f)
   }
 }
 
-// dense interior operator of the coarse level (with the coarse-level kappa
-// when present) and its FP64 inverse, on the device; the handle's inverse is
-// replaced once the new one is known to be good
-void build_dense_coarse(tps_handle *h)
+// dense interior operator of the coarse level (with the coarse-level kappa when
+// present) assembled cell by cell on the host in FP64, and its inverse
+std::vector<double> dense_coarse_host(const tps_handle *h)
 {
-  const int k = h->k, n = h->n_coarse, dim = h->dim, m1 = n * k - 1;
+  const int k = h->k, n = h->n_coarse, N1 = n * k + 1, dim = h->dim;
+  const double hh = 1.0 / n, s = stiffness_scale(dim, hh);
+  const int np = k + 1;
+  const int m1 = N1 - 2;
   const int ni = dim == 3 ? m1 * m1 * m1 : m1 * m1;
-  const size_t bytes = sizeof(double) * static_cast<size_t>(ni) * ni, nt = h->D.cmass.size();
-  if (!h->coarse_tab.p) {
-    h->coarse_tab.alloc(sizeof(double) * (2 * nt + 1));
-    double *t = h->coarse_tab.as<double>();
-    TPS_CUDA(cudaMemcpy(t, h->D.cmass.data(), sizeof(double) * nt, cudaMemcpyHostToDevice));
-    TPS_CUDA(cudaMemcpy(t + nt, h->D.clap.data(), sizeof(double) * nt, cudaMemcpyHostToDevice));
+  // interior index of a global coarse DoF (-1 on the boundary)
+  auto interior = [&](int x, int y, int z) -> int {
+    if (x < 1 || x > N1 - 2 || y < 1 || y > N1 - 2) return -1;
+    if (dim == 3 && (z < 1 || z > N1 - 2)) return -1;
+    return (x - 1) + (y - 1) * m1 + (dim == 3 ? (z - 1) * m1 * m1 : 0);
+  };
+  std::vector<double> A(static_cast<size_t>(ni) * ni, 0.0);
+  const int ncell = dim == 3 ? n * n * n : n * n;
+  const int csz = dim == 3 ? np * np * np : np * np;
+  for (int c = 0; c < ncell; ++c) {
+    const int cx = c % n, cy = (c / n) % n, cz = dim == 3 ? c / (n * n) : 0;
+    const double kc = h->has_kappa ? h->kappa_host[0][c] : 1.0;
+    for (int a = 0; a < csz; ++a) {
+      const int ax = a % np, ay = (a / np) % np, az = dim == 3 ? a / (np * np) : 0;
+      const int ia = interior(cx * k + ax, cy * k + ay, cz * k + az);
+      if (ia < 0) continue;
+      for (int b2 = 0; b2 < csz; ++b2) {
+        const int bx = b2 % np, by = (b2 / np) % np, bz = dim == 3 ? b2 / (np * np) : 0;
+        const int ib = interior(cx * k + bx, cy * k + by, cz * k + bz);
+        if (ib < 0) continue;
+        const double mx = h->D.cmass[ax * np + bx], my = h->D.cmass[ay * np + by];
+        const double lx = h->D.clap[ax * np + bx], ly = h->D.clap[ay * np + by];
+        double v;
+        if (dim == 2) {
+          v = ly * mx + my * lx;
+        } else {
+          const double mz = h->D.cmass[az * np + bz], lz = h->D.clap[az * np + bz];
+          v = lz * my * mx + mz * ly * mx + mz * my * lx;
+        }
+        A[static_cast<size_t>(ia) * ni + ib] += kc * s * v;
+      }
+    }
   }
-  for (DevBuf &w : h->coarse_work)
-    if (!w.p) w.alloc(bytes);
-  if (!h->coarse_inv.p) h->coarse_inv.alloc(bytes);
-  double *t = h->coarse_tab.as<double>(), *a = h->coarse_work[0].as<double>();
+  // explicit inverse (coarse systems hold at most a few thousand DoFs)
+  std::vector<double> inv;
+  try {
+    inv = spd_inverse(A, ni);
+  } catch (const std::runtime_error &) {
+    throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
+  }
+  return inv;
+}
+
+// the same on the device, into the handle's inverse, which is replaced once the
+// new one is known to be good
+void dense_coarse_device(tps_handle *h, int ni)
+{
+  const int k = h->k, n = h->n_coarse, dim = h->dim;
+  const size_t n2 = static_cast<size_t>(ni) * ni, nt = h->D.cmass.size();
+  if (!h->coarse_inv.p) h->coarse_inv.alloc(sizeof(double) * n2);
+  if (!h->coarse_work.p) h->coarse_work.alloc(sizeof(double) * (2 * nt + 1 + 2 * n2));
+  double *t = h->coarse_work.as<double>(), *a = t + 2 * nt + 1;
   int *bad = reinterpret_cast<int *>(t + 2 * nt);
+  std::vector<double> tab(h->D.cmass);
+  tab.insert(tab.end(), h->D.clap.begin(), h->D.clap.end());
+  tab.push_back(0.0);  // the flag
+  TPS_CUDA(cudaMemcpy(t, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
   const CoarseOperator op{dim, k, n, t, t + nt, h->has_kappa ? h->kappa_dev[0][0]->as<double>() : nullptr,
                           stiffness_scale(dim, 1.0 / n)};
   TPS_CUDA(launch_assemble_coarse(a, op, ni, nullptr));
-  TPS_CUDA(launch_spd_inverse(a, h->coarse_work[1].as<double>(), ni, bad, nullptr));
+  TPS_CUDA(launch_spd_inverse(a, a + n2, ni, bad, nullptr));
   int failed = 0;
   TPS_CUDA(cudaMemcpy(&failed, bad, sizeof(int), cudaMemcpyDeviceToHost));
   if (failed) throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
-  TPS_CUDA(cudaMemcpy(h->coarse_inv.p, a, bytes, cudaMemcpyDeviceToDevice));
+  TPS_CUDA(cudaMemcpyAsync(h->coarse_inv.p, a, sizeof(double) * n2, cudaMemcpyDeviceToDevice, nullptr));
   TPS_CUDA(cudaStreamSynchronize(nullptr));  // any stream may read it from here on
-  if (bytes > (size_t(32) << 20))
-    for (DevBuf &w : h->coarse_work) w.release();
+  if (h->coarse_work.bytes > (size_t(64) << 20)) h->coarse_work.release();
+}
+
+// A small coarse operator is inverted on the host, where a new handle then
+// needs no device memory and no launches for it before its first V-cycle
+// (creating and closing one, us, host / device: 25 rows 77 / 1210, 125 rows 392 /
+// 5371, 361 rows 4734 / 2801, 1331 rows 79431 / 4958); with a coefficient, whose
+// updates rebuild it into memory that is there (about 60 us), from 48 rows on
+// the device.
+void build_dense_coarse(tps_handle *h)
+{
+  const int m1 = h->n_coarse * h->k - 1, dim = h->dim;
+  const int ni = dim == 3 ? m1 * m1 * m1 : m1 * m1;
+  if (ni <= (h->has_kappa ? 48 : 160)) {
+    h->coarse_inv_host = dense_coarse_host(h);
+    if (h->coarse_inv.p)
+      TPS_CUDA(cudaMemcpy(h->coarse_inv.p, h->coarse_inv_host.data(), sizeof(double) * h->coarse_inv_host.size(),
+                          cudaMemcpyHostToDevice));
+  } else {
+    dense_coarse_device(h, ni);
+  }
   h->n_int_coarse = ni;
   h->coarse_coord.resize(3 * static_cast<size_t>(ni));
   for (int i = 0; i < ni; ++i) {
@@ -400,6 +466,13 @@ VcycleVectors &vcycle_vectors(tps_handle *h, int p)
                                  h->coarse_coord[3 * i + 2] * lc.sz);
     V.coarse_idx.alloc(sizeof(int) * ni);
     TPS_CUDA(cudaMemcpy(V.coarse_idx.p, gidx.data(), sizeof(int) * ni, cudaMemcpyHostToDevice));
+  }
+  if (h->dense_coarse && !h->coarse_inv.p) {
+    DevBuf inv;
+    inv.alloc(sizeof(double) * h->coarse_inv_host.size());
+    TPS_CUDA(cudaMemcpy(inv.p, h->coarse_inv_host.data(), inv.bytes, cudaMemcpyHostToDevice));
+    std::swap(h->coarse_inv.p, inv.p);
+    std::swap(h->coarse_inv.bytes, inv.bytes);
   }
   if (h->dense_coarse && p == 1) {
     V.coarse_inv.alloc(sizeof(float) * static_cast<size_t>(h->n_int_coarse) * h->n_int_coarse);

@@ -83,6 +83,17 @@ struct DegreeTables {
 template <int K, typename T>
 __constant__ DegreeTables<K, T> c_tables;
 
+// Tables that are indexed per lane, in global memory (one copy per degree and
+// precision, uploaded with the constant ones).
+template <int K, typename T>
+struct LaneTables {
+  T rlam3[Dims<K>::M * Dims<K>::M * Dims<K>::M];  // 1 / (lambda_x + lambda_y + lambda_z), z-major
+  T rlam2[Dims<K>::M * Dims<K>::M];               // 1 / (lambda_y + lambda_x), [y mode][x mode]
+  T prows2[2 * Dims<K>::N1 * Dims<K>::M];         // rows 1..2k-1 of the patch mass and stiffness, [matrix][entry][row]
+};
+template <int K, typename T>
+__device__ LaneTables<K, T> g_lane_tables;
+
 // Geometry of one level: n cells per direction, N1 = n*k+1 DoFs per direction.
 struct LevelGeom {
   int n;       // cells per direction
