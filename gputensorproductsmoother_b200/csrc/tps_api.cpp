@@ -1095,19 +1095,22 @@ void autotune_levels(tps_handle *h, int p, cudaStream_t s)
   TPS_CUDA(cudaMemsetAsync(V.su.back()->p, 0, V.su.back()->bytes, s));
 }
 
+// whether work on s goes into a graph instead of running now
+bool is_capturing(cudaStream_t s)
+{
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the legacy stream while another one is captured
+  return true;
+}
+
 // The row-padded copies of tps_smoother_step's vectors and their TMA views,
-// allocated at the finest level's size by the first call that wants them (so
-// captured calls keep valid pointers).  False where there is no memory for
-// them, or the stream is capturing (which allows no allocation) before they
-// exist: the sweep then reads the caller's vectors.
-bool stage_vectors(tps_handle *h, int p, cudaStream_t s)
+// allocated at the finest level's size by the first call that wants them.
+// False where there is no memory for them: the sweep then reads the caller's
+// vectors.
+bool stage_vectors(tps_handle *h, int p)
 {
   if (!h->stage_maps[p].empty()) return true;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return false;
-  }
   const size_t es = p == 0 ? sizeof(double) : sizeof(float);
   const VecLayout top = padded_layout(h, h->n_levels - 1, es);
   const size_t bytes = es * static_cast<size_t>(top.sz) * top.N1;
@@ -1130,7 +1133,10 @@ bool stage_vectors(tps_handle *h, int p, cudaStream_t s)
   return true;
 }
 
-// tps_smoother_step on caller vectors by way of row-padded copies
+// tps_smoother_step on caller vectors by way of row-padded copies.  Never
+// inside a stream capture: the copies are shared by all calls of the handle, and
+// nothing orders a graph's replays, or two branches of one capture, after each
+// other's use of them.
 void staged_smoother_step(tps_handle *h, int level, int p, void *x, const void *b, bool zero_init, bool reverse,
                           cudaStream_t s)
 {
@@ -1139,12 +1145,7 @@ void staged_smoother_step(tps_handle *h, int level, int p, void *x, const void *
   const VecLayout lay = padded_layout(h, level, es);
   const PadMap pm = make_padmap(lay.N1, lay.sy);
   void *px = h->stage_x[p].p, *pb = h->stage_b[p].p;
-  // the copies are shared by all calls of the handle: a call on another
-  // stream waits for the last one (calls inside a capture are ordered by it)
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  const bool free_running = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
-  if (!free_running) cudaGetLastError();
-  if (free_running && s != h->stage_stream[p]) TPS_CUDA(cudaStreamWaitEvent(s, h->stage_done[p], 0));
+  if (s != h->stage_stream[p]) TPS_CUDA(cudaStreamWaitEvent(s, h->stage_done[p], 0));
   if (zero_init) {
     TPS_CUDA(cudaMemsetAsync(px, 0, es * static_cast<size_t>(lay.sz) * lay.N1, s));
     TPS_CUDA(launch_pad_rows(pb, b, nullptr, nullptr, pm, N, es, s));
@@ -1153,10 +1154,8 @@ void staged_smoother_step(tps_handle *h, int level, int p, void *x, const void *
   }
   smoother_sweep(h, level, p, lay, px, pb, reverse, zero_init, &h->stage_maps[p][level], s);
   TPS_CUDA(launch_unpad_rows(x, px, pm, N, es, s));
-  if (free_running) {
-    TPS_CUDA(cudaEventRecord(h->stage_done[p], s));
-    h->stage_stream[p] = s;
-  }
+  TPS_CUDA(cudaEventRecord(h->stage_done[p], s));
+  h->stage_stream[p] = s;
 }
 
 // Whether a level's 3D sweep on caller vectors pays for the copies: their rows
@@ -1523,7 +1522,7 @@ int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *
       return;
     }
     const int p = dt_index(dtype);
-    if (stage_pays(h, level) && stage_vectors(h, p, s)) {
+    if (stage_pays(h, level) && !is_capturing(s) && stage_vectors(h, p)) {
       staged_smoother_step(h, level, p, x, b, zero_init != 0, reverse != 0, s);
       return;
     }

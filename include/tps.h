@@ -82,9 +82,9 @@ int tps_laplace_vmult(tps_handle *h, int level, int dtype, void *dst, const void
  * reverse=1 runs the colours in reverse order (symmetric post-smoothing).
  * 3D sweeps at degree >= 3 or of at least 2e5 DoFs work on row-padded copies
  * of x and b: the first such call of a precision allocates two vectors of the
- * finest level's size, which the handle keeps (without memory for them, or
- * first called inside a stream capture, the sweep reads x and b in place;
- * same results). */
+ * finest level's size, which the handle keeps.  Without memory for them, and
+ * inside a stream capture (whose replays may run beside other sweeps of the
+ * handle), the sweep works on x and b in place; same results. */
 int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *b,
                       int zero_init, int reverse, void *stream);
 

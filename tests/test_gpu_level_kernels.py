@@ -91,6 +91,40 @@ def test_smoother_3d_copies_serve_every_level_and_stream(cuda, oracle):
     Q.close()
 
 
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_captured_sweeps_share_nothing(cuda, dtype):
+    """Sweeps captured after the handle has its copies: two branches of one
+    graph, replayed while the handle sweeps other vectors on another stream."""
+    P = tps.PoissonProblem(3, 4, 8)
+    S = tps.PatchSmoother(P)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x0, b = ([torch.rand(P.n_dofs(), device="cuda", dtype=dtype, generator=gen) for _ in range(3)] for _ in range(2))
+    ref = [v.clone() for v in x0]
+    for v, w in zip(ref, b):  # the copies exist from here on
+        for _ in range(4):
+            S.step(v, w)
+    x = [v.clone() for v in x0]
+    fork, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        fork.wait_stream(torch.cuda.current_stream())
+        for _ in range(2):
+            S.step(x[0], b[0])
+            with torch.cuda.stream(fork):
+                S.step(x[1], b[1])
+        torch.cuda.current_stream().wait_stream(fork)
+    for _ in range(2):
+        g.replay()
+        with torch.cuda.stream(other):
+            S.step(x[2], b[2])
+            S.step(x[2], b[2])
+    torch.cuda.synchronize()
+    for v, w in zip(x, ref):
+        assert torch.equal(v, w)
+    P.close()
+
+
 def test_captured_solves_serve_any_vectors(cuda):
     """The captured CG iteration and the batch's graph are built once and read
     the caller's vectors from device memory: repeated solves with new right-hand
