@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
@@ -231,8 +232,8 @@ struct tps_handle {
   // the finest-level size and their TMA views per level, [FP64, FP32]
   DevBuf stage_x[2], stage_b[2];
   std::vector<SmootherMaps> stage_maps[2];
-  cudaEvent_t stage_done[2] = {nullptr, nullptr};  // end of the last use, and its stream
-  cudaStream_t stage_stream[2] = {nullptr, nullptr};
+  cudaEvent_t stage_done[2] = {nullptr, nullptr};  // end of the last use
+  std::mutex stage_mutex;  // a call's wait, launches and record follow one another
   DevBuf dense_inv[2];  // Exact variant: reference-cell interior patch inverse [FP64, FP32]
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -1145,7 +1146,10 @@ void staged_smoother_step(tps_handle *h, int level, int p, void *x, const void *
   const VecLayout lay = padded_layout(h, level, es);
   const PadMap pm = make_padmap(lay.N1, lay.sy);
   void *px = h->stage_x[p].p, *pb = h->stage_b[p].p;
-  if (s != h->stage_stream[p]) TPS_CUDA(cudaStreamWaitEvent(s, h->stage_done[p], 0));
+  // always after the last use, also where the stream's handle is the last
+  // one's: a new stream can have a destroyed one's handle, and the per-thread
+  // default streams share theirs
+  TPS_CUDA(cudaStreamWaitEvent(s, h->stage_done[p], 0));
   if (zero_init) {
     TPS_CUDA(cudaMemsetAsync(px, 0, es * static_cast<size_t>(lay.sz) * lay.N1, s));
     TPS_CUDA(launch_pad_rows(pb, b, nullptr, nullptr, pm, N, es, s));
@@ -1155,7 +1159,6 @@ void staged_smoother_step(tps_handle *h, int level, int p, void *x, const void *
   smoother_sweep(h, level, p, lay, px, pb, reverse, zero_init, &h->stage_maps[p][level], s);
   TPS_CUDA(launch_unpad_rows(x, px, pm, N, es, s));
   TPS_CUDA(cudaEventRecord(h->stage_done[p], s));
-  h->stage_stream[p] = s;
 }
 
 // Whether a level's 3D sweep on caller vectors pays for the copies: their rows
@@ -1522,9 +1525,12 @@ int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *
       return;
     }
     const int p = dt_index(dtype);
-    if (stage_pays(h, level) && !is_capturing(s) && stage_vectors(h, p)) {
-      staged_smoother_step(h, level, p, x, b, zero_init != 0, reverse != 0, s);
-      return;
+    if (stage_pays(h, level) && !is_capturing(s)) {
+      std::lock_guard<std::mutex> lock(h->stage_mutex);
+      if (stage_vectors(h, p)) {
+        staged_smoother_step(h, level, p, x, b, zero_init != 0, reverse != 0, s);
+        return;
+      }
     }
     if (zero_init) TPS_CUDA(cudaMemsetAsync(x, 0, (p == 0 ? 8 : 4) * g.N, s));
     smoother_sweep(h, level, p, lex_layout(h, level), x, b, reverse != 0, zero_init != 0, nullptr, s);

@@ -91,6 +91,53 @@ def test_smoother_3d_copies_serve_every_level_and_stream(cuda, oracle):
     Q.close()
 
 
+def test_smoother_3d_copies_with_one_stream_handle(cuda):
+    """Sweeps of two vector pairs on streams that share one handle: the
+    per-thread default streams (handle 2) of two threads in turn, without a
+    wait between them."""
+    import threading
+    from gputensorproductsmoother_b200 import _lib as L
+    P = tps.PoissonProblem(3, 4, 16)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x0, b = ([torch.rand(P.n_dofs(), device="cuda", dtype=torch.float64, generator=gen) for _ in range(2)]
+             for _ in range(2))
+    ref = [v.clone() for v in x0]
+    for v, w in zip(ref, b):
+        for _ in range(6):
+            tps.PatchSmoother(P).step(v, w)
+    x = [v.clone() for v in x0]
+    torch.cuda.synchronize()
+
+    def sweeps(i):
+        for _ in range(3):
+            L.check(L.lib().tps_smoother_step(P.handle, P.n_levels - 1, L.TPS_F64, x[i].data_ptr(), b[i].data_ptr(),
+                                              0, 0, 2), P.handle)
+
+    # the streams live on while their threads wait
+    go, done = [threading.Event() for _ in range(5)], [threading.Event() for _ in range(4)]
+
+    def worker(i):
+        for r in (i, i + 2):
+            go[r].wait()
+            sweeps(i)
+            done[r].set()
+        go[4].wait()
+
+    ts = [threading.Thread(target=worker, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for r in range(4):
+        go[r].set()
+        assert done[r].wait(60)
+    torch.cuda.synchronize()
+    go[4].set()
+    for t in ts:
+        t.join()
+    for v, w in zip(x, ref):
+        assert torch.equal(v, w)
+    P.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 def test_captured_sweeps_share_nothing(cuda, dtype):
     """Sweeps captured after the handle has its copies: two branches of one
