@@ -214,6 +214,7 @@ struct tps_handle {
   // CUDA graph of one CG iteration
   cudaGraphExec_t graph = nullptr;
   int graph_key = -1;
+  uint64_t settings = 0;  // counts the changes after which a captured solve is out of date
   int tc_passes = 1;  // tensor-core smoother: 1 TF32 pass, 3 the three-term TF32 split
   cudaStream_t own_stream = nullptr;  // used by tps_solve_host
   DevBuf host_b, host_x;              // device staging of tps_solve_host (kept, so its graph stays valid)
@@ -255,6 +256,15 @@ struct tps_handle {
 };
 
 namespace {
+
+// after a change of what a solve launches: its captured forms (this handle's CG
+// iteration, the graph of a batch that owns the handle) are captured anew
+void settings_changed(tps_handle *h)
+{
+  ++h->settings;
+  if (h->graph) cudaGraphExecDestroy(h->graph);
+  h->graph = nullptr;
+}
 
 int dt_index(int dtype)
 {
@@ -1679,10 +1689,7 @@ int tps_set_kappa(tps_handle *h, const double *kappa, int rebuild_coarse)
       build_dense_coarse(h);
       if (h->vc[1].ready) round_coarse_inverse(h);
     }
-    if (h->graph) {  // re-captured on the next solve
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-    }
+    settings_changed(h);
   });
 }
 
@@ -1774,10 +1781,7 @@ int tps_set_smoother_variant(tps_handle *h, int dtype, int level, int variant)
     h->sm_variant[p][level] = variant;
     if (static_cast<int>(h->sm_explicit[p].size()) != h->n_levels) h->sm_explicit[p].assign(h->n_levels, 0);
     h->sm_explicit[p][level] = 1;
-    if (h->graph) {  // later solves re-capture with the chosen kernel
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-    }
+    settings_changed(h);
   });
 }
 
@@ -1795,10 +1799,7 @@ int tps_set_smoother_kind(tps_handle *h, int kind, double damping)
       ensure_additive_scratch(h, 1);
     }
     h->sm_kind = kind;
-    if (h->graph) {  // a captured CG iteration holds the previous smoothing
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-    }
+    settings_changed(h);
   });
 }
 
@@ -1822,10 +1823,7 @@ int tps_set_operator_layers(tps_handle *h, int dtype, int level, int layers)
       throw ApiError(TPS_ERR_INVALID, "operator layers must be 0 (default), 1, 2, 4, 8 or 16");
     if (static_cast<int>(h->op_layers[p].size()) != h->n_levels) h->op_layers[p].assign(h->n_levels, 0);
     h->op_layers[p][level] = layers;
-    if (h->graph) {  // later solves re-capture with the chosen tile depth
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-    }
+    settings_changed(h);
   });
 }
 
@@ -1846,10 +1844,7 @@ int tps_autotune(tps_handle *h, int dtype, int *ppb_per_level)
     if (!h->own_stream) TPS_CUDA(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
     autotune_levels(h, p, h->own_stream);
     TPS_CUDA(cudaStreamSynchronize(h->own_stream));
-    if (h->graph) {  // later solves re-capture with the chosen kernels
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-    }
+    settings_changed(h);
     if (ppb_per_level)
       for (int l = 0; l < h->n_levels; ++l)
         ppb_per_level[l] = h->kt->smoother_ppb(h->dim, p == 0 ? 0 : 1, h->sm_variant[p][l]);
@@ -2106,6 +2101,7 @@ struct tps_batch {
   // what the instantiated graph was built for
   int k_prec = -1, k_sym = -1, k_max = -1;
   double k_tol = -1.0;
+  std::vector<uint64_t> k_settings;  // per system
   DevBuf sc_ptrs, iters, active, bnorm, hist;
   DevBuf systems, results;    // BatchSystem and BatchResult per system
   void *host = nullptr;       // pinned: the results, then the residual histories
@@ -2177,8 +2173,8 @@ std::vector<cudaGraphNode_t> capture_deps(cudaStream_t s, cudaGraph_t *g)
 }
 
 // The graph works on the systems' own vectors and finds the caller's in the
-// loaded scalars, so it is built once per precision, colour order, max_iter
-// and tolerance.
+// loaded scalars, so it is built once per precision, colour order, max_iter,
+// tolerance and settings of the systems.
 void batch_build(tps_batch *B, const tps_solve_opts &o, cudaStream_t s)
 {
   const int n = static_cast<int>(B->sys.size());
@@ -2286,6 +2282,8 @@ void batch_build(tps_batch *B, const tps_solve_opts &o, cudaStream_t s)
   B->k_sym = o.symmetric != 0;
   B->k_max = o.max_iter;
   B->k_tol = o.rel_tol;
+  B->k_settings.clear();
+  for (const tps_handle *h : B->sys) B->k_settings.push_back(h->settings);
 }
 
 template <typename F>
@@ -2417,8 +2415,9 @@ int tps_batch_solve(tps_batch *B, const tps_solve_opts *opts, const double *cons
       TPS_CUDA(cudaStreamWaitEvent(B->own, B->fork_ev, 0));
       s = B->own;
     }
-    const bool same = B->exec && B->k_prec == opts->precision && B->k_sym == (opts->symmetric != 0) &&
-                      B->k_max == opts->max_iter && B->k_tol == opts->rel_tol;
+    bool same = B->exec && B->k_prec == opts->precision && B->k_sym == (opts->symmetric != 0) &&
+                B->k_max == opts->max_iter && B->k_tol == opts->rel_tol;
+    for (int i = 0; same && i < n; ++i) same = B->k_settings[i] == B->sys[i]->settings;
     if (!same) batch_build(B, *opts, s);
     BatchIo io{};
     for (int i = 0; i < n; ++i) {

@@ -333,7 +333,8 @@ int tps_get_smoother_variant(tps_handle *h, int dtype, int level, int *variant);
  * conditional node per system, parallel branches) followed by a check kernel;
  * the host waits once, when every system has converged or reached max_iter.
  * The instantiated graph is reused, on any stream and for any vectors, while
- * precision, symmetric, max_iter and rel_tol stay the same. */
+ * precision, symmetric, max_iter and rel_tol stay the same; a setting changed
+ * on one of the systems (tps_batch_system) applies from the next solve on. */
 typedef struct tps_batch tps_batch;
 int tps_batch_create(const tps_problem *problems, int n_systems, tps_batch **out);
 int tps_batch_destroy(tps_batch *b);

@@ -58,6 +58,65 @@ def test_batch_max_iter_and_zero_rhs(cuda):
     B.close()
 
 
+def test_batch_takes_up_settings_of_its_systems(cuda):
+    """A setting changed on one of the systems between two solves applies to
+    the second, as it does to a batch that never solved before."""
+    import ctypes
+    from gputensorproductsmoother_b200 import _lib as L
+    lib, systems = L.lib(), [(3, 3, 8), (3, 3, 8), (3, 2, 12)]
+    rhs = [interior_random(d, n * k + 1, 30 + i) for i, (d, k, n) in enumerate(systems)]
+
+    def handle(B, i):
+        h = ctypes.c_void_p()
+        assert lib.tps_batch_system(B._h, i, ctypes.byref(h)) == L.TPS_OK
+        return h
+
+    changes = [lambda B: lib.tps_set_smoother_kind(handle(B, 0), L.SMOOTHER_ADDITIVE, 0.0),
+               lambda B: lib.tps_set_operator_layers(handle(B, 1), L.TPS_F64, 2, 1),
+               lambda B: lib.tps_set_smoother_variant(handle(B, 2), L.TPS_F32, 1, 0),
+               lambda B: lib.tps_set_smoother_kind(handle(B, 0), L.SMOOTHER_FUSED, 0.0)]
+    # explicit choices everywhere, so that no timing decides a handle's kernels
+    def new_batch():
+        B = tps.BatchSolver(systems)
+        for i in range(3):
+            for lv in range(3):
+                assert lib.tps_set_smoother_variant(handle(B, i), L.TPS_F32, lv, 1) == L.TPS_OK
+        return B
+
+    B = new_batch()
+    iters = []
+    for step in range(len(changes) + 1):
+        if step:
+            assert changes[step - 1](B) == L.TPS_OK
+        C = new_batch()
+        for f in changes[:step]:
+            assert f(C) == L.TPS_OK
+        got, reps = B.solve(rhs, precision="fp32")
+        want, wreps = C.solve(rhs, precision="fp32")
+        iters.append([r.iterations for r in reps])
+        assert iters[-1] == [r.iterations for r in wreps], step
+        for g, w in zip(got, want):
+            assert torch.equal(g, w), step
+        C.close()
+    assert iters[1][0] > iters[0][0] and iters[1][1:] == iters[0][1:] and iters[-1] == iters[0]
+    B.close()
+
+
+def test_batch_of_the_largest_number_of_systems(cuda):
+    """256 systems in one graph; every one its own solution."""
+    systems = [(2, 1 + i % 3, 4 + 2 * (i % 5)) for i in range(256)]
+    B = tps.BatchSolver(systems)
+    rhs = [interior_random(d, n * k + 1, i) for i, (d, k, n) in enumerate(systems)]
+    xs, reps = B.solve(rhs, precision="fp64")
+    for i in (0, 97, 255):
+        P = tps.PoissonProblem(*systems[i])
+        x1, r1 = tps.MultigridSolvers(P).solve_cg(rhs[i], precision="fp64")
+        assert reps[i].iterations == r1.iterations
+        assert (xs[i] - x1).abs().max().item() <= 1e-12 * x1.abs().max().item()
+        P.close()
+    B.close()
+
+
 def test_autotune_keeps_results(cuda):
     """The kernel variants only regroup independent patches of a colour: the
     autotuned sweep is bit-identical to the default one."""
