@@ -94,17 +94,11 @@ struct Ks3 {
   static constexpr size_t BYTES = sizeof(T) * ELEMS;
 };
 
-// a compile-time integer as a function argument
-template <int V>
-struct IntC {
-  static constexpr int value = V;
-};
-
 // rows Y0+1 .. Y0+NY (y) and 1..k (z) of the cell product of one thread:
 // acc[z][y] = L_z M_y TA + M_z (L_y TA + M_y TB); ta, tb point at the cell's
 // outermost (z, y) entry of this x node, dz and dy step inward
-template <int K, typename T, int Y0, int NY>
-__device__ __forceinline__ void ks3_planes(const T *ta, const T *tb, int dz, int dy, T (&acc)[K][NY])
+template <int K, typename T, int Y0, int NY, int NA>
+__device__ __forceinline__ void ks3_planes(const T *ta, const T *tb, int dz, int dy, T (&acc)[K][NA])
 {
   constexpr int NP = K + 1;
   const DegreeTables<K, T> &c = c_tables<K, T>;
@@ -228,26 +222,25 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
     const int dz = oz ? -S::TZ : S::TZ;
     T *c0 = TA + (oz ? (2 * K - 1) * S::CP : 0) + (oy ? (2 * K - 1) * S::CR : 0) + (ox ? 2 * K - 1 - d : d);
     const int cz = oz ? -S::CP : S::CP, cy = oy ? -S::CR : S::CR;
-    // the y halves are stored from the outside inward: both step forward
-    auto run = [&](auto y0c, auto nyc) {
-      constexpr int Y0 = decltype(y0c)::value, NY = decltype(nyc)::value;
-      T acc[K][NY];
-      if (cell_lane) ks3_planes<K, T, Y0, NY>(TA + base, TB + base, dz, 2, acc);
-      sync();  // TA and TB are read
-      if (cell_lane) {
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-          for (int q = 0; q < NY; ++q) c0[i * cz + (Y0 + q) * cy] = kap * acc[i][q];
-      }
-    };
-    if constexpr (S::YS == 1) {
-      run(IntC<0>{}, IntC<K>{});
-    } else {
+    // the y halves are stored from the outside inward: both step forward.  A
+    // group has its own rows of constant-bank coefficients, so its own code; the
+    // barrier between the reads and the writes is one for the CTA
+    T acc[K][S::YR];
+    if (cell_lane) {
       if (grp == 0)
-        run(IntC<0>{}, IntC<S::YR>{});
-      else
-        run(IntC<S::YR>{}, IntC<K - S::YR>{});
+        ks3_planes<K, T, 0, S::YR>(TA + base, TB + base, dz, 2, acc);
+      else if constexpr (S::YS == 2)
+        ks3_planes<K, T, S::YR, K - S::YR>(TA + base, TB + base, dz, 2, acc);
+    }
+    sync();  // TA and TB are read
+    if (cell_lane) {
+      c0 += grp * S::YR * cy;
+#pragma unroll
+      for (int q = 0; q < S::YR; ++q)
+        if (q < K - S::YR || grp == 0) {
+#pragma unroll
+          for (int i = 0; i < K; ++i) c0[i * cz + q * cy] = kap * acc[i][q];
+        }
     }
   }
   sync();
