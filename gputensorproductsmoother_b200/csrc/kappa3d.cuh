@@ -162,6 +162,8 @@ __global__ void __launch_bounds__(Ks3<K, T>::NT)
   const bool cell_lane = gl < 8 * K;
   const int o = cell_lane ? gl / K : 0, d = cell_lane ? gl - o * K : 0;
   const int ox = o & 1, oy = (o >> 1) & 1, oz = o >> 2;
+  // before the wait: no kernel writes kappa (read after it, a sweep took 1.5 to 2
+  // us more: Q4 48^3 FP64 613.6 / 615.1, Q7 16^3 208.3 / 210.6)
   const T kap = s * kc[ox + oy * n + int64_t(oz) * n * n];
   T kd[8];
   if (tid < 27) {

@@ -1,8 +1,12 @@
 // Kernel launches with programmatic dependent launch (sm_90 and later).
 //
 // Every kernel of this library starts with griddep_wait(), before its first
-// global-memory access, and every launch carries the programmatic stream
-// serialization attribute.  A kernel may then be launched, and its CTAs
+// access to memory that a kernel may have written, and every launch carries the
+// programmatic stream serialization attribute.  What only the host writes, by
+// copies that have completed when the entry point returns, may be read before
+// it: the tables (c_tables, g_lane_tables; the 2D smoother's rows) and the
+// coefficient (the kappa 3D smoother).  A kernel that came to write one of them
+// would have to be followed by readers that wait first.  A kernel may then be launched, and its CTAs
 // scheduled, while the previous kernel in the stream is still finishing;
 // griddep_wait() returns once that grid has completed and its memory
 // operations are visible.  Inside the CUDA graphs of the solvers the launch

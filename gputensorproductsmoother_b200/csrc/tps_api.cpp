@@ -626,6 +626,8 @@ void set_kappa_levels(tps_handle *h, const double *kappa_fine)
     const std::vector<float> f(kh[l].begin(), kh[l].end());
     TPS_CUDA(cudaMemcpy(h->kappa_dev[1][l]->p, f.data(), sizeof(float) * nc, cudaMemcpyHostToDevice));
   }
+  // complete on return: kernels read the coefficient ahead of their wait (launch.cuh)
+  TPS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   h->kappa_host = std::move(kh);
 }
 
@@ -1458,6 +1460,7 @@ int tps_create(const tps_problem *pb, tps_handle **out)
     if (!h->kt) throw ApiError(TPS_ERR_UNSUPPORTED, "degree not compiled in");
     h->D = make_degree_data(pb->degree);
     TPS_CUDA(h->kt->upload(h->D));
+    TPS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // complete on return, as kappa is
     if (pb->kappa) {
       h->has_kappa = true;
       set_kappa_levels(h.get(), pb->kappa);
