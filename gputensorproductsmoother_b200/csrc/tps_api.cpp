@@ -194,7 +194,7 @@ struct tps_handle {
   int n_int_coarse = 0;
   DevBuf coarse_inv;                    // n_int^2, FP64
   std::vector<double> coarse_inv_host;  // a small one, until the first V-cycle needs it on the device
-  DevBuf coarse_work;                   // reference-cell mass and stiffness, the inversion's flag, its two matrices
+  DevBuf coarse_work;                   // with kappa: reference-cell matrices, the inversion's flag, its two matrices
   std::vector<int> coarse_coord;        // (x, y, z) of each interior coarse DoF
   VcycleVectors vc[2];  // [0] FP64, [1] FP32
   std::vector<int> sm_variant[2];  // per level: 3D smoother patches-per-batch variant (autotuned)
@@ -378,7 +378,9 @@ void dense_coarse_device(tps_handle *h, int ni)
   if (failed) throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
   TPS_CUDA(cudaMemcpyAsync(h->coarse_inv.p, a, sizeof(double) * n2, cudaMemcpyDeviceToDevice, nullptr));
   TPS_CUDA(cudaStreamSynchronize(nullptr));  // any stream may read it from here on
-  if (h->coarse_work.bytes > (size_t(64) << 20)) h->coarse_work.release();
+  // kept for the updates of a coefficient, which then cannot run out of memory
+  // half-way; a constant one is inverted once
+  if (!h->has_kappa) h->coarse_work.release();
 }
 
 // A small coarse operator is inverted on the host, where a new handle then

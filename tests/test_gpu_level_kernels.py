@@ -272,6 +272,46 @@ def test_dense_coarse_inverse(cuda, dim, k, n, varying):
     P.close()
 
 
+def test_kappa_update_needs_no_memory(cuda):
+    """A new coefficient is taken up whole where device memory has run out, also
+    with a large dense coarse level (2601 rows, 54 MB a matrix)."""
+    from gputensorproductsmoother_b200 import _lib as L
+    kap = np.exp(np.random.default_rng(3).normal(0.0, 0.5, (2, 26 ** 2)))
+    P, Q = (tps.PoissonProblem(2, 2, 26, n_coarse=26, kappa=kap[i]) for i in range(2))
+    b = torch.rand(P.n_dofs(), dtype=torch.float64, device="cuda")
+    got, want = P.new_vector(), P.new_vector()
+    tps.MultigridSolvers(P).vmult(got, b, precision="fp64")
+    L.lib().tps_inject_alloc_failure(1)
+    try:
+        P.set_kappa(kap[1])
+    finally:
+        L.lib().tps_inject_alloc_failure(0)
+    for f in (lambda p, v: tps.MultigridSolvers(p).vmult(v, b, precision="fp64"),
+              lambda p, v: tps.LaplaceOperator(p).vmult(v, b)):
+        f(P, got)
+        f(Q, want)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    P.close()
+    Q.close()
+
+
+def test_constant_coarse_level_holds_no_workspace(cuda):
+    """A constant coefficient's coarse operator is inverted once: the handle
+    keeps its inverse (1331 rows, 14.2 MB), not what the inversion worked in."""
+    make = lambda: tps.PoissonProblem(3, 4, 3, n_coarse=3)
+    make().close()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    Ps = [make() for _ in range(8)]
+    torch.cuda.synchronize()
+    held = (free0 - torch.cuda.mem_get_info()[0]) / len(Ps)
+    # one matrix, in pieces of at most 2 MB of a shared pool, and small buffers
+    assert held < 1.5 * 8 * 1331 ** 2, held
+    for P in Ps:
+        P.close()
+
+
 # the varying-coefficient operator and smoother: tiles with remainders, several
 # layer chunks, every degree (the cells' rows are split over two thread groups
 # in FP64 from degree 5 on); padded rows are covered by the V-cycles elsewhere
