@@ -141,6 +141,11 @@ struct DevBuf {
     bytes = b;
     TPS_CUDA(cudaMemset(p, 0, b));
   }
+  void swap(DevBuf &o)
+  {
+    std::swap(p, o.p);
+    std::swap(bytes, o.bytes);
+  }
   template <typename T>
   T *as() const { return static_cast<T *>(p); }
 };
@@ -192,8 +197,8 @@ struct tps_handle {
   // coarse level: single vertex patch (n_coarse == 2) or dense solve
   bool dense_coarse = false;
   int n_int_coarse = 0;
-  DevBuf coarse_inv;                    // n_int^2, FP64
-  std::vector<double> coarse_inv_host;  // a small one, until the first V-cycle needs it on the device
+  DevBuf coarse_inv;                    // n_int^2, FP64; with kappa, and as long as a V-cycle may need it
+  std::vector<double> coarse_inv_host;  // one inverted on the host
   DevBuf coarse_work;                   // with kappa: reference-cell matrices, the inversion's flag, its two matrices
   std::vector<int> coarse_coord;        // (x, y, z) of each interior coarse DoF
   VcycleVectors vc[2];  // [0] FP64, [1] FP32
@@ -361,7 +366,8 @@ void dense_coarse_device(tps_handle *h, int ni)
 {
   const int k = h->k, n = h->n_coarse, dim = h->dim;
   const size_t n2 = static_cast<size_t>(ni) * ni, nt = h->D.cmass.size();
-  if (!h->coarse_inv.p) h->coarse_inv.alloc(sizeof(double) * n2);
+  DevBuf first;  // becomes the handle's inverse
+  if (!h->coarse_inv.p) first.alloc(sizeof(double) * n2);
   if (!h->coarse_work.p) h->coarse_work.alloc(sizeof(double) * (2 * nt + 1 + 2 * n2));
   double *t = h->coarse_work.as<double>(), *a = t + 2 * nt + 1;
   int *bad = reinterpret_cast<int *>(t + 2 * nt);
@@ -376,8 +382,10 @@ void dense_coarse_device(tps_handle *h, int ni)
   int failed = 0;
   TPS_CUDA(cudaMemcpy(&failed, bad, sizeof(int), cudaMemcpyDeviceToHost));
   if (failed) throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
-  TPS_CUDA(cudaMemcpyAsync(h->coarse_inv.p, a, sizeof(double) * n2, cudaMemcpyDeviceToDevice, nullptr));
+  TPS_CUDA(cudaMemcpyAsync(first.p ? first.p : h->coarse_inv.p, a, sizeof(double) * n2, cudaMemcpyDeviceToDevice,
+                           nullptr));
   TPS_CUDA(cudaStreamSynchronize(nullptr));  // any stream may read it from here on
+  if (first.p) h->coarse_inv.swap(first);
   // kept for the updates of a coefficient, which then cannot run out of memory
   // half-way; a constant one is inverted once
   if (!h->has_kappa) h->coarse_work.release();
@@ -408,6 +416,20 @@ void build_dense_coarse(tps_handle *h)
     h->coarse_coord[3 * i + 1] = 1 + (i / m1) % m1;
     h->coarse_coord[3 * i + 2] = dim == 3 ? 1 + i / (m1 * m1) : 0;
   }
+}
+
+// the FP64 inverse into device memory, where it is not there
+void coarse_inverse_on_device(tps_handle *h)
+{
+  if (h->coarse_inv.p) return;
+  if (h->coarse_inv_host.empty()) {
+    dense_coarse_device(h, h->n_int_coarse);
+    return;
+  }
+  DevBuf inv;
+  inv.alloc(sizeof(double) * h->coarse_inv_host.size());
+  TPS_CUDA(cudaMemcpy(inv.p, h->coarse_inv_host.data(), inv.bytes, cudaMemcpyHostToDevice));
+  h->coarse_inv.swap(inv);
 }
 
 // the FP32 V-cycle's rounded copy of the dense coarse inverse
@@ -480,16 +502,15 @@ VcycleVectors &vcycle_vectors(tps_handle *h, int p)
     V.coarse_idx.alloc(sizeof(int) * ni);
     TPS_CUDA(cudaMemcpy(V.coarse_idx.p, gidx.data(), sizeof(int) * ni, cudaMemcpyHostToDevice));
   }
-  if (h->dense_coarse && !h->coarse_inv.p) {
-    DevBuf inv;
-    inv.alloc(sizeof(double) * h->coarse_inv_host.size());
-    TPS_CUDA(cudaMemcpy(inv.p, h->coarse_inv_host.data(), inv.bytes, cudaMemcpyHostToDevice));
-    std::swap(h->coarse_inv.p, inv.p);
-    std::swap(h->coarse_inv.bytes, inv.bytes);
-  }
-  if (h->dense_coarse && p == 1) {
-    V.coarse_inv.alloc(sizeof(float) * static_cast<size_t>(h->n_int_coarse) * h->n_int_coarse);
-    round_coarse_inverse(h);
+  if (h->dense_coarse) {
+    coarse_inverse_on_device(h);
+    if (p == 1) {
+      V.coarse_inv.alloc(sizeof(float) * static_cast<size_t>(h->n_int_coarse) * h->n_int_coarse);
+      round_coarse_inverse(h);
+      // a constant coefficient's FP64 inverse is held for FP64 V-cycles only
+      // (the first one after FP32 ones forms it again, with the same bits)
+      if (!h->has_kappa && !h->vc[0].ready) h->coarse_inv.release();
+    }
   }
   V.ready = true;
   return V;

@@ -308,7 +308,25 @@ def test_constant_coarse_level_holds_no_workspace(cuda):
     held = (free0 - torch.cuda.mem_get_info()[0]) / len(Ps)
     # one matrix, in pieces of at most 2 MB of a shared pool, and small buffers
     assert held < 1.5 * 8 * 1331 ** 2, held
+    # FP32 V-cycles need the rounded inverse alone; a later FP64 one is that of
+    # a handle that had no FP32 ones
+    b = torch.rand(Ps[0].n_dofs(), dtype=torch.float64, device="cuda")
     for P in Ps:
+        tps.MultigridSolvers(P).vmult(P.new_vector(), b, precision="fp32")
+    torch.cuda.synchronize()
+    held = (free0 - torch.cuda.mem_get_info()[0]) / len(Ps)
+    assert held < 0.8 * 8 * 1331 ** 2, held
+    Q = make()
+    z = [P.new_vector() for P in (Q, Ps[0], Ps[0])]
+    for P, v, precision in ((Q, z[0], "fp64"), (Ps[0], z[1], "fp64"), (Ps[0], z[2], "fp32")):
+        tps.MultigridSolvers(P).vmult(v, b, precision=precision)
+    tps.MultigridSolvers(Q).vmult(Q.new_vector(), b, precision="fp32")
+    w = [Q.new_vector() for _ in range(2)]
+    for v, precision in zip(w, ("fp64", "fp32")):
+        tps.MultigridSolvers(Q).vmult(v, b, precision=precision)
+    torch.cuda.synchronize()
+    assert torch.equal(z[0], z[1]) and torch.equal(w[0], z[0]) and torch.equal(w[1], z[2])
+    for P in Ps + [Q]:
         P.close()
 
 
