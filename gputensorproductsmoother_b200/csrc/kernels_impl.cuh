@@ -82,9 +82,12 @@ cudaError_t upload_one(const DegreeData &D)
       lt.prows2[j * M + r] = static_cast<T>(D.pmass[(r + 1) * N1 + j]);
       lt.prows2[(N1 + j) * M + r] = static_cast<T>(D.plap[(r + 1) * N1 + j]);
     }
-  const cudaError_t e = cudaMemcpyToSymbol(g_lane_tables<K, T>, &lt, sizeof(lt));
+  // queued one after the other (the host's copies are staged when a call
+  // returns); upload waits once
+  const cudaError_t e = cudaMemcpyToSymbolAsync(g_lane_tables<K, T>, &lt, sizeof(lt), 0, cudaMemcpyHostToDevice,
+                                                cudaStreamLegacy);
   if (e != cudaSuccess) return e;
-  return cudaMemcpyToSymbol(c_tables<K, T>, &t, sizeof(t));
+  return cudaMemcpyToSymbolAsync(c_tables<K, T>, &t, sizeof(t), 0, cudaMemcpyHostToDevice, cudaStreamLegacy);
 }
 
 template <int DIM, typename T>
@@ -199,6 +202,8 @@ cudaError_t upload(const DegreeData &D)
 #endif
   if (e == cudaSuccess) e = set_attributes<double>();
   if (e == cudaSuccess) e = set_attributes<float>();
+  // complete on return: kernels read tables ahead of their wait (launch.cuh)
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
   return e;
 }
 

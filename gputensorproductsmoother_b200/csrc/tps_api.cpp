@@ -1483,7 +1483,6 @@ int tps_create(const tps_problem *pb, tps_handle **out)
     if (!h->kt) throw ApiError(TPS_ERR_UNSUPPORTED, "degree not compiled in");
     h->D = make_degree_data(pb->degree);
     TPS_CUDA(h->kt->upload(h->D));
-    TPS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // complete on return, as kappa is
     if (pb->kappa) {
       h->has_kappa = true;
       set_kappa_levels(h.get(), pb->kappa);
