@@ -391,17 +391,19 @@ void dense_coarse_device(tps_handle *h, int ni)
   if (!h->has_kappa) h->coarse_work.release();
 }
 
-// A small coarse operator is inverted on the host, where a new handle then
-// needs no device memory and no launches for it before its first V-cycle
-// (creating and closing one, us, host / device: 25 rows 77 / 1210, 125 rows 392 /
-// 5371, 361 rows 4734 / 2801, 1331 rows 79431 / 4958); with a coefficient, whose
-// updates rebuild it into memory that is there (about 60 us), from 48 rows on
-// the device.
+// A small coarse operator is inverted on the host, a larger one on the device.
+// Measured, us, host / device (minimum of 3 times 10 calls).  Creating and
+// closing a handle with a constant coefficient, where the device's part is mostly
+// its allocations: 25 rows 45 / 690, 125 rows 285 / 793, 196 rows 785 / 947, 216 rows
+// 986 / 926, 256 rows 1463 / 904, 512 rows 10067 / 1776.  An update of a varying one:
+// 49 rows 59 / 98, 81 rows 106 / 124, 100 rows 154 / 161, 121 rows 223 / 164, 125 rows
+// 283 / 166, 196 rows 720 / 254, 512 rows 8387 / 532 (its creation 100 rows 782 / 828,
+// 121 rows 862 / 817).
 void build_dense_coarse(tps_handle *h)
 {
   const int m1 = h->n_coarse * h->k - 1, dim = h->dim;
   const int ni = dim == 3 ? m1 * m1 * m1 : m1 * m1;
-  if (ni <= (h->has_kappa ? 48 : 160)) {
+  if (ni <= (h->has_kappa ? 110 : 200)) {
     h->coarse_inv_host = dense_coarse_host(h);
     if (h->coarse_inv.p)
       TPS_CUDA(cudaMemcpy(h->coarse_inv.p, h->coarse_inv_host.data(), sizeof(double) * h->coarse_inv_host.size(),

@@ -245,10 +245,11 @@ def test_assemble_tiles(cuda, oracle, dim, k, n):
 
 # one level: the V-cycle is the dense inverse alone.  Sizes below, at and just
 # past the inversion's 32-column blocks and 64-entry tiles, up to its largest
-# ones; cond(A) is at most 4 (2 n k)^2, so that a backward-stable inverse
+# ones, and the last on the host and the first on the device; cond(A) is at most 4 (2 n k)^2, so that a backward-stable inverse
 # leaves a residual of a few cond * 2^-53
 @pytest.mark.parametrize("dim,k,n", [(2, 1, 2), (2, 1, 3), (2, 2, 3), (2, 1, 7), (2, 1, 9), (2, 4, 2), (3, 1, 5),
-                                     (2, 1, 33), (2, 1, 34), (3, 4, 3), (3, 1, 16), (2, 2, 32)])
+                                     (2, 1, 33), (2, 1, 34), (3, 4, 3), (3, 1, 16), (2, 2, 32), (2, 1, 11), (2, 1, 12),
+                                     (2, 3, 5), (3, 1, 7)])
 @pytest.mark.parametrize("varying", [False, True])
 def test_dense_coarse_inverse(cuda, dim, k, n, varying):
     kap = None
