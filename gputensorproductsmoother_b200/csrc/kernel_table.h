@@ -67,7 +67,7 @@ struct KernelTable {
   cudaError_t (*encode_maps[2])(const VecLayout &l, void *x, const void *b, SmootherMaps *out);
   // fine += P coarse (interior fine DoFs); geometry of the COARSE level
   cudaError_t (*prolong[2][2])(const LevelGeomH &coarse, const VecLayout &lc, const VecLayout &lf,
-                               void *fine, const void *coarse_v, void *tmp, cudaStream_t);
+                               void *fine, const void *coarse_v, cudaStream_t);
   // coarse (+)= R fine on interior coarse DoFs; geometry of the COARSE level;
   // zero (may be null, not with add): a coarse vector to zero on the interior
   cudaError_t (*restrict_[2][2])(const LevelGeomH &coarse, const VecLayout &lc,
@@ -108,7 +108,7 @@ struct KernelTable {
   int (*smoother_ppb)(int dim, int dtype, int variant);
   // FP64 fine += P coarse with the coarse boundary values used ([dim - 2])
   cudaError_t (*prolong_nb[2])(const LevelGeomH &coarse, const VecLayout &lc, const VecLayout &lf,
-                               void *fine, const void *coarse_v, void *tmp, cudaStream_t);
+                               void *fine, const void *coarse_v, cudaStream_t);
   // separate-kernel smoother variants (cross-checks of the fused kernels), per
   // colour: r_I = (b - A x)_I on the interiors of the colour's patches, and
   // x_I <- omega (x_I + A_II^{-1} r_I) with the fast diagonalisation (inv

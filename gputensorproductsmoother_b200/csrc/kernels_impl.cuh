@@ -624,17 +624,15 @@ cudaError_t encode_maps(const VecLayout &l, void *x, const void *b, SmootherMaps
 
 template <int DIM, typename T, bool MASK>
 cudaError_t prolong_impl(const LevelGeomH &gc, const VecLayout &lc, const VecLayout &lf, void *fine,
-                         const void *coarse, void *tmp, cudaStream_t s)
+                         const void *coarse, cudaStream_t s)
 {
   const int N1c = gc.N1, N1f = 2 * gc.n * K + 1;
   if constexpr (DIM == 2) {
     const unsigned gxy = ceil_div(gc.n, ProlTile<K, T>::C);
-    (void)tmp;
-    TPS_LAUNCH((prolong_xy_kernel<K, T, XYOut::AddInterior>), dim3(gxy, gxy, 1), XYTile<K>::NT, 0, s,
-        static_cast<T *>(fine), static_cast<const T *>(coarse), N1c, N1f, lc.sy, 0, lf.sy, 0, 0, MASK ? 1 : 0);
+    TPS_LAUNCH((prolong2d_kernel<K, T, MASK>), dim3(gxy, gxy), XYTile<K>::NT, 0, s, static_cast<T *>(fine),
+        static_cast<const T *>(coarse), N1c, N1f, lc.sy, lf.sy);
   } else {
     using S = Prol3<K, T>;
-    (void)tmp;
     TPS_LAUNCH((prolong3d_kernel<K, T, MASK>), dim3(ceil_div(gc.n, S::TX), ceil_div(gc.n, S::TY), gc.n), S::NT,
         S::BYTES, s, static_cast<T *>(fine), static_cast<const T *>(coarse), N1c, N1f, lc.sy, lc.sz, lf.sy, lf.sz);
   }
@@ -643,18 +641,18 @@ cudaError_t prolong_impl(const LevelGeomH &gc, const VecLayout &lc, const VecLay
 
 template <int DIM, typename T>
 cudaError_t prolong(const LevelGeomH &gc, const VecLayout &lc, const VecLayout &lf, void *fine,
-                    const void *coarse, void *tmp, cudaStream_t s)
+                    const void *coarse, cudaStream_t s)
 {
-  return prolong_impl<DIM, T, true>(gc, lc, lf, fine, coarse, tmp, s);
+  return prolong_impl<DIM, T, true>(gc, lc, lf, fine, coarse, s);
 }
 
 // FP64 prolongation that reads the coarse boundary values (the FMG
 // prolongation of the solution); fine interior DoFs += P coarse
 template <int DIM>
 cudaError_t prolong_nb(const LevelGeomH &gc, const VecLayout &lc, const VecLayout &lf, void *fine,
-                       const void *coarse, void *tmp, cudaStream_t s)
+                       const void *coarse, cudaStream_t s)
 {
-  return prolong_impl<DIM, double, false>(gc, lc, lf, fine, coarse, tmp, s);
+  return prolong_impl<DIM, double, false>(gc, lc, lf, fine, coarse, s);
 }
 
 template <int DIM, typename T>
@@ -737,16 +735,16 @@ cudaError_t kappa_laplace(const LevelGeomH &g, const VecLayout &l, void *dst, co
     else
       TPS_LAUNCH((kappa_laplace3d_kernel<K, T, false>), grid, S::NT, S::BYTES, st, static_cast<T *>(dst),
           static_cast<const T *>(src), nullptr, static_cast<const T *>(kappa), g.n, l.sy, l.sz, layers, sc);
-    return cudaGetLastError();
+  } else {
+    const int64_t n = l.sy * g.N1;
+    cudaError_t e = cudaMemsetAsync(dst, 0, sizeof(T) * n, st);
+    if (e != cudaSuccess) return e;
+    e = cell_sweep<DIM, T, false>(g, l, static_cast<T *>(dst), static_cast<const T *>(src),
+                                  static_cast<const T *>(kappa), stiffness_scale(DIM, g.h), st);
+    if (e != cudaSuccess) return e;
+    TPS_LAUNCH((finish_residual_kernel<DIM, T>), 1184, 256, 0, st,
+        static_cast<T *>(dst), mode == 1 ? static_cast<const T *>(rhs) : nullptr, g.N1, l.sy, l.sz);
   }
-  const int64_t n = l.sy * g.N1;
-  cudaError_t e = cudaMemsetAsync(dst, 0, sizeof(T) * n, st);
-  if (e != cudaSuccess) return e;
-  e = cell_sweep<DIM, T, false>(g, l, static_cast<T *>(dst), static_cast<const T *>(src),
-                                static_cast<const T *>(kappa), stiffness_scale(DIM, g.h), st);
-  if (e != cudaSuccess) return e;
-  TPS_LAUNCH((finish_residual_kernel<DIM, T>), 1184, 256, 0, st,
-      static_cast<T *>(dst), mode == 1 ? static_cast<const T *>(rhs) : nullptr, g.N1, l.sy, l.sz);
   return cudaGetLastError();
 }
 

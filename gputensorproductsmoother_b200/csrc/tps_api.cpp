@@ -228,7 +228,6 @@ struct tps_handle {
   DevBuf pipe_b[2], pipe_x[2];
   cudaEvent_t pipe_in[2] = {nullptr, nullptr}, pipe_done[2] = {nullptr, nullptr}, pipe_out[2] = {nullptr, nullptr};
   std::vector<std::unique_ptr<DevBuf>> fmg_sol, fmg_res;  // FMG: FP64 per level (lexicographic)
-  DevBuf fmg_tmp;                                        // FMG: FP64 transfer scratch
   DevBuf adj_g, adj_lam;                                 // tps_adjoint: its right-hand side and lambda
   DevBuf var_r[2];      // separate-kernel smoother variants: residual of the finest-level size
   DevBuf var_acc[2];    // additive step: the summed patch solves
@@ -778,8 +777,7 @@ void vcycle_rec(tps_handle *h, int level, int p, bool symmetric, cudaStream_t s,
   TPS_CUDA(h->kt->restrict_[di][p](h->lv[level - 1], lc, lay, V.d[level - 1]->p, V.t[level]->p,
                                    V.tmp[level]->p, 0, zero_with(h, p, level - 1), s));
   vcycle_rec(h, level - 1, p, symmetric, s, tc);
-  TPS_CUDA(h->kt->prolong[di][p](h->lv[level - 1], lc, lay, V.su[level]->p, V.su[level - 1]->p,
-                                 V.tmp[level]->p, s));
+  TPS_CUDA(h->kt->prolong[di][p](h->lv[level - 1], lc, lay, V.su[level]->p, V.su[level - 1]->p, s));
   level_smooth(h, level, p, lay, V.su[level]->p, V.d[level]->p, symmetric, false, &V.maps[level], s, tcl);
 }
 
@@ -1249,16 +1247,12 @@ void fmg(tps_handle *h, int precision, int n_cycles, const double *const *rhs, c
   if (h->fmg_sol.size() != static_cast<size_t>(h->n_levels)) {
     // built aside and kept only once every allocation succeeded
     std::vector<std::unique_ptr<DevBuf>> sol, res;
-    size_t tmp = 0;
     for (int l = 0; l <= L; ++l) {
       sol.emplace_back(new DevBuf);
       res.emplace_back(new DevBuf);
       if (l < L) sol[l]->alloc(sizeof(double) * h->lv[l].N);
       res[l]->alloc(sizeof(double) * h->lv[l].N);
-      if (l > 0 && dim == 3)
-        tmp = std::max(tmp, sizeof(double) * static_cast<size_t>(h->lv[l].N1) * h->lv[l - 1].N1 * h->lv[l - 1].N1);
     }
-    if (tmp) h->fmg_tmp.alloc(tmp);
     h->fmg_sol = std::move(sol);
     h->fmg_res = std::move(res);
   }
@@ -1278,7 +1272,7 @@ void fmg(tps_handle *h, int precision, int n_cycles, const double *const *rhs, c
     double *res = h->fmg_res[l]->as<double>();
     if (bnd && bnd[l - 1]) TPS_CUDA(launch_copy_boundary(solc, bnd[l - 1], dim, gc.N1, 8, s));
     TPS_CUDA(cudaMemsetAsync(sol, 0, sizeof(double) * g.N, s));
-    TPS_CUDA(h->kt->prolong_nb[dim - 2](gc, lex_layout(h, l - 1), lex_layout(h, l), sol, solc, h->fmg_tmp.p, s));
+    TPS_CUDA(h->kt->prolong_nb[dim - 2](gc, lex_layout(h, l - 1), lex_layout(h, l), sol, solc, s));
     TPS_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * g.N, s));
     level_laplace(h, l, 0, lex_layout(h, l), res, sol, rhs[l], 1, s);
     TPS_CUDA(launch_to_vcycle(V.d[l]->p, zero_with(h, p, l), input_kind(precision), padmap(l), res, g.N, s));
@@ -1633,10 +1627,8 @@ int tps_prolongate_add(tps_handle *h, int to_level, int dtype, void *fine, const
     const int p = dt_index(dtype);
     if (!fine || !coarse) throw ApiError(TPS_ERR_INVALID, "null vector");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    VcycleVectors &V = vcycle_vectors(h, p);
     TPS_CUDA(h->kt->prolong[h->dim - 2][p](h->lv[to_level - 1], lex_layout(h, to_level - 1),
-                                           lex_layout(h, to_level), fine, coarse,
-                                           V.tmp[to_level]->p, s));
+                                           lex_layout(h, to_level), fine, coarse, s));
   });
 }
 

@@ -13,9 +13,10 @@
 // written as gathers (no atomics, deterministic):
 //   fine(i)   = sum_j P1(i_z,j_z) P1(i_y,j_y) P1(i_x,j_x) coarse(j)
 //   coarse(j) = sum_i P1(i_z,j_z) P1(i_y,j_y) P1(i_x,j_x) fine(i)
-// A 3D transfer is one 1D pass along z plus one 2D pass per xy-plane; the
-// intermediate (fine z x coarse y x coarse x, a quarter of the fine level)
-// lives in a per-level scratch buffer.
+// A prolongation is one pass over tiles of the fine level.  A 3D restriction is
+// one 2D pass per xy-plane plus one 1D pass along z; the intermediate (fine z x
+// coarse y x coarse x, a quarter of the fine level) lives in a per-level scratch
+// buffer.
 #pragma once
 
 #include "ptx.cuh"
@@ -35,9 +36,9 @@ struct XYTile {
   static constexpr int NT = 256;
 };
 
-// prolongation: 8 coarse cells per CTA for FP32 at k <= 4 (measured 58 -> 53
-// us at 3D Q4 64^3), else 4 (k <= 4; FP64 measured 99 us with 4, 115 with 8)
-// or 2
+// 2D prolongation: coarse cells per CTA and direction.  Measured, us per
+// prolongate-and-add in FP32, 8 / 4 cells: Q1 1024^2 12.3 / 13.1, Q4 512^2 12.5 /
+// 12.4; FP64 tiles of 8 cells need more than 48 KB at degree 4.
 template <int K, typename T>
 struct ProlTile {
   static constexpr int C = (sizeof(T) == 4 && K <= 4) ? 8 : K <= 4 ? 4 : 2;
@@ -79,14 +80,12 @@ __device__ __forceinline__ void restr_cell(const T (&v)[4 * K + 1], T (&out)[K])
 }
 
 // ---------------------------------------------------------------------------
-// xy pass, prolongation: coarse plane (N1c x N1c) -> fine plane (N1f x N1f).
-// Rows are in_sy / out_sy apart; in/out advance by the plane strides per
-// blockIdx.z (plane index offset by plane0).  Coarse boundary entries are read as zero when mask_in != 0.
-template <int K, typename T, XYOut OUT>
+// 2D prolongation: fine interior += P coarse for a tile of C x C coarse cells
+// (rows c_sy / f_sy apart).  Coarse boundary entries read as zero (MASK) or as
+// they are.
+template <int K, typename T, bool MASK>
 __global__ void __launch_bounds__(XYTile<K>::NT)
-    prolong_xy_kernel(T *__restrict__ out, const T *__restrict__ in, int N1c, int N1f,
-                      int64_t in_sy, int64_t in_plane, int64_t out_sy, int64_t out_plane,
-                      int plane0, int mask_in)
+    prolong2d_kernel(T *__restrict__ fine, const T *__restrict__ coarse, int N1c, int N1f, int64_t c_sy, int64_t f_sy)
 {
   griddep_wait();  // programmatic launch: the previous kernel's writes are visible
   constexpr int C = ProlTile<K, T>::C, NT = XYTile<K>::NT;
@@ -94,25 +93,15 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
   constexpr int WO = 2 * K * C;  // fine outputs per direction
   __shared__ T sIn[WI * WI];
   __shared__ T sX[WI * WO];
-  const int plane = plane0 + blockIdx.z;
-  const T *inp = in + plane * in_plane;
-  T *outp = out + plane * out_plane;
   const int cx0 = blockIdx.x * C, cy0 = blockIdx.y * C;
-  // In add mode with at most one y-stage task per thread (FP64 tiles) the
-  // task's current fine values are loaded first, so that the loads' latency
-  // overlaps the coarse tile load and the x stage (measured at 3D Q4 64^3:
-  // FP64 prolongation 0.094 -> 0.085 ms; with the two tasks of the FP32 tiles
-  // the extra registers cost more than the overlap gained, 0.050 -> 0.068 ms,
-  // so those tiles stage the values in shared memory instead, below)
-  constexpr bool PREFETCH = OUT == XYOut::AddInterior && WO * C <= NT;
-  // The other add-mode tiles (FP32) stage the current fine values of the
-  // tile in shared memory by asynchronous copies, issued right after the
-  // coarse tile's, so that the read-modify-write of the fine level waits on
-  // no load at the end (3D Q4 64^3 mixed solve 12.35 -> 12.23 ms; the
-  // coarse tile by asynchronous copies as well, 12.37 -> 12.35)
-  constexpr bool STAGE_CUR = OUT == XYOut::AddInterior && !PREFETCH;
-  __shared__ T sCur[STAGE_CUR ? WO * WO : 1];
-  T cur[1][2 * K];
+  // The current fine values are loaded first, so that their latency overlaps
+  // the coarse tile's load and the x stage: into registers where a thread has
+  // at most one y-stage task (FP64 tiles), else by asynchronous copies into
+  // shared memory, issued right after the coarse tile's (the registers of two
+  // tasks cost more than the overlap gained).
+  constexpr bool PREFETCH = WO * C <= NT;
+  __shared__ T sCur[PREFETCH ? 1 : WO * WO];
+  T cur[2 * K];
   if constexpr (PREFETCH) {
     const int t = threadIdx.x;
     const int xx = t % WO, c = t / WO;
@@ -121,7 +110,7 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
     for (int f = 0; f < 2 * K; ++f) {
       const int gy = 2 * K * (cy0 + c) + f;
       const bool interior = t < WO * C && gx > 0 && gx < N1f - 1 && gy > 0 && gy < N1f - 1;
-      cur[0][f] = interior ? outp[gx + gy * out_sy] : T(0);
+      cur[f] = interior ? fine[gx + gy * f_sy] : T(0);
     }
   }
   {
@@ -130,19 +119,19 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
       const int lx = e % WI, ly = e / WI;
       const int gx = cx0 * K + lx, gy = cy0 * K + ly;
       const bool bnd = gx == 0 || gx == N1c - 1 || gy == 0 || gy == N1c - 1;
-      const bool ok = gx < N1c && gy < N1c && !(mask_in && bnd);
-      cp_async_zfill_s<sizeof(T)>(s_in + static_cast<uint32_t>(sizeof(T) * e), ok ? inp + gx + gy * in_sy : inp,
+      const bool ok = gx < N1c && gy < N1c && !(MASK && bnd);
+      cp_async_zfill_s<sizeof(T)>(s_in + static_cast<uint32_t>(sizeof(T) * e), ok ? coarse + gx + gy * c_sy : coarse,
                                   ok ? static_cast<uint32_t>(sizeof(T)) : 0u);
     }
     cp_async_commit();
   }
-  if constexpr (STAGE_CUR) {
+  if constexpr (!PREFETCH) {
     const uint32_t s_cur = smem_u32(sCur);
     for (int e = threadIdx.x; e < WO * WO; e += NT) {
       const int xx = e % WO, yy = e / WO;
       const int gx = 2 * K * cx0 + xx, gy = 2 * K * cy0 + yy;
       const bool ok = gx < N1f && gy < N1f;
-      cp_async_zfill_s<sizeof(T)>(s_cur + static_cast<uint32_t>(sizeof(T) * e), ok ? outp + gx + gy * out_sy : outp,
+      cp_async_zfill_s<sizeof(T)>(s_cur + static_cast<uint32_t>(sizeof(T) * e), ok ? fine + gx + gy * f_sy : fine,
                                   ok ? static_cast<uint32_t>(sizeof(T)) : 0u);
     }
     cp_async_commit();
@@ -160,40 +149,22 @@ __global__ void __launch_bounds__(XYTile<K>::NT)
 #pragma unroll
     for (int f = 0; f < 2 * K; ++f) sX[y * WO + c * 2 * K + f] = o[f];
   }
-  if constexpr (STAGE_CUR) cp_async_wait_all();  // this thread's share of the fine tile
+  if constexpr (!PREFETCH) cp_async_wait_all();  // this thread's share of the fine tile
   __syncthreads();
-  // y stage: fine rows of the tile, added to (or stored into) the fine plane
-  auto y_task = [&](int t, const T (&add)[2 * K]) {
+  for (int t = threadIdx.x; t < WO * C; t += NT) {
     const int xx = t % WO, c = t / WO;
     T v[K + 1], o[2 * K];
 #pragma unroll
     for (int b = 0; b <= K; ++b) v[b] = sX[(c * K + b) * WO + xx];
     prol_cell<K, T>(v, o);
     const int gx = 2 * K * cx0 + xx;
-    if (gx >= N1f) return;
+    if (gx == 0 || gx >= N1f - 1) continue;
 #pragma unroll
     for (int f = 0; f < 2 * K; ++f) {
       const int gy = 2 * K * (cy0 + c) + f;
-      if (gy >= N1f) continue;
-      const int64_t gi = gx + gy * out_sy;
-      const bool interior = gx > 0 && gx < N1f - 1 && gy > 0 && gy < N1f - 1;
-      if constexpr (PREFETCH) {
-        if (interior) outp[gi] = add[f] + o[f];
-      } else if constexpr (STAGE_CUR) {
-        if (interior) outp[gi] = sCur[(2 * K * c + f) * WO + xx] + o[f];
-      } else if constexpr (OUT == XYOut::AddInterior) {
-        if (interior) outp[gi] += o[f];
-      } else if constexpr (OUT == XYOut::SetInterior) {
-        if (interior) outp[gi] = o[f];
-      } else {
-        outp[gi] = o[f];
-      }
+      if (gy == 0 || gy >= N1f - 1) continue;
+      fine[gx + gy * f_sy] = (PREFETCH ? cur[f] : sCur[(2 * K * c + f) * WO + xx]) + o[f];
     }
-  };
-  if constexpr (PREFETCH) {
-    if (threadIdx.x < WO * C) y_task(threadIdx.x, cur[0]);
-  } else {
-    for (int t = threadIdx.x; t < WO * C; t += NT) y_task(t, cur[0]);
   }
 }
 
