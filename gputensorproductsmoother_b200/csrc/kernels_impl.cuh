@@ -413,14 +413,17 @@ cudaError_t smoother(const LevelGeomH &g, const VecLayout &l, void *x, const voi
 }
 
 // Whether a level's sweep runs as one launch of one cluster (sweep_cluster.cuh).
-// Measured, us per sweep, one launch / a launch per colour:
+// Measured, us per sweep, one launch / a launch per colour (50 sweeps, best of 5):
 //   2D, one CTA (at most 7 warps of patches in the largest colour): FP64 Q1 16^2
-//   5.0 / 13.3, Q2 8^2 6.9 / 9.6, Q2 16^2 8.4 / 9.4, Q5 8^2 11.0 / 15.9, Q7 4^2 14.1 /
-//   18.6; FP32 Q2 16^2 7.4 / 9.8, Q4 8^2 7.8 / 9.7; but with 8 warps Q7 8^2 FP64
-//   19.3 / 18.9, and with the barrier of several CTAs Q3 32^2 15.7 / 10.4;
-//   3D, a patch per CTA up to 8 CTAs: FP32 Q4 4^3 18.2 / 29.9, Q4 8^3 22.5 / 31.1,
-//   Q1 8^3 13.5 / 27.4, Q7 4^3 47.6 / 61.4; FP64 Q3 8^3 25.7 / 27.0, Q4 4^3 26.3 /
-//   30.8; but Q4 8^3 FP64 35.7 / 32.6, Q5 8^3 FP32 42.9 / 38.5.
+//   7.0 / 8.7, Q2 8^2 7.1 / 8.9, Q2 16^2 9.3 / 9.4, Q5 8^2 11.5 / 15.1, Q7 6^2 15.8 /
+//   18.3; FP32 Q2 16^2 7.0 / 8.7, Q4 8^2 7.7 / 9.2; with 8 and more warps Q7 8^2 FP64
+//   19.3 / 18.4, Q4 12^2 13.0 / 11.4, Q3 16^2 11.9 / 10.1;
+//   3D, a patch per CTA up to 8 CTAs, 8 patches (4^3): FP64 Q3 21.6 / 25.5, Q4 26.4 /
+//   31.5, Q5 48.8 / 48.4 (3^3 50.7 / 48.1), Q6 47.0 / 71.7, Q7 91.4 / 93.5; FP32 Q4 18.3 /
+//   30.2, Q7 47.8 / 62.3;
+//   27 patches (6^3): FP64 Q3 23.8 / 25.6, Q4 32.2 / 31.7; FP32 Q4 20.7 / 29.9, Q5 42.0 /
+//   37.1; 64 patches (8^3): FP64 Q2 20.0 / 22.7, Q3 32.3 / 26.8, Q4 47.8 / 32.8; FP32 Q1
+//   13.8 / 27.4, Q3 25.2 / 25.2, Q4 29.5 / 30.8.
 // Two cells per direction have one patch and one launch as it is.
 bool sweep_pays(int dim, int dtype, int n)
 {
@@ -429,7 +432,7 @@ bool sweep_pays(int dim, int dtype, int n)
   if (dim == 2) return ceil_div(int64_t(c) * c, 32 / (2 * K - 1)) <= 7;
   const int count = c * c * c;
   if (n < 10 && count <= 8) return !(K == 5 && dtype == 0);
-  return n < 10 && count <= 64 && (K <= 3 || (K == 4 && dtype == 1));
+  return n < 10 && (K <= 2 || (K == 3 && (dtype == 1 || count <= 27)) || (K == 4 && dtype == 1));
 }
 
 template <int DIM, typename T>

@@ -318,9 +318,12 @@ int tps_set_smoother_variant(tps_handle *h, int dtype, int level, int variant);
  *     at least 4096 patches;
  *   - otherwise quarter CTA batches at degrees 2 and 3, and the default batch
  *     at other degrees.
- * On the smallest levels (at most 8 patches per colour, 64 at degrees up to 3
- * and at degree 4 in FP32) a sweep is one launch of its own kernel, with the same
- * results, unless tps_set_smoother_variant chose a variant for the level. */
+ * On the smallest levels a sweep is one launch of its own kernel, with the same
+ * results, unless tps_set_smoother_variant chose a variant for the level.  3D:
+ * 3 to 9 cells per direction at degrees 1 and 2, at degree 3 (FP64: up to 7) and
+ * at degree 4 in FP32; 3 to 5 otherwise, except FP64 at degree 5.  2D: from 3
+ * cells on, while the largest colour, (n/2)^2 patches of n cells per direction,
+ * fills at most 7 warps of 32 / (2k-1) patches each. */
 int tps_get_smoother_variant(tps_handle *h, int dtype, int level, int *variant);
 
 /* ---- batched solves (no reference counterpart) ----------------------------
