@@ -743,10 +743,14 @@ bool tc_pays(const tps_handle *h, int level)
 
 // The V-cycle's solution vector of a level, to be zeroed with the stores that
 // write its right-hand side; null where vcycle_rec fills it itself.  A fill
-// costs its own launch and the overlap of its neighbours' (2D Q2 64^2 solve
-// 1181 us with fills, 1036 without); vectors beyond 16 MB cost more as one more
-// stream of the writing kernel than as a fill (Q4 64^3 solve 10.21 against
-// 10.26 ms).
+// costs its own launch and the overlap of its neighbours'; a large vector costs
+// more as one more stream of the writing kernel.  Measured, us per CG solve:
+//   stores on every level / fills on every level: 2D Q2 64^2 1036 / 1181, 3D Q3 32^3
+//   FP32 1873 / 1906, Q4 32^3 2652 / 2686, 2D Q5 384^2 2756 / 2830, 3D Q4 64^3 10105 /
+//   10068 (FP64 16582 / 16535);
+//   the finest level alone, store / fill: Q4 32^3 FP64 (17 MB) 3548 / 3551, Q3 48^3 FP64
+//   (24 MB) 4326 / 4322, Q4 48^3 FP32 (29 MB) 5089 / 5083, Q2 96^3 FP32 (29 MB) 7324 / 7309.
+// From 16 to 30 MB the two are equal to 0.2 %, so the line is not critical.
 void *zero_with(const tps_handle *h, int p, int level)
 {
   const DevBuf &su = *h->vc[p].su[level];
