@@ -222,7 +222,7 @@ struct tps_handle {
   uint64_t settings = 0;  // counts the changes after which a captured solve is out of date
   int tc_passes = 1;  // tensor-core smoother: 1 TF32 pass, 3 the three-term TF32 split
   cudaStream_t own_stream = nullptr;  // used by tps_solve_host
-  DevBuf host_b, host_x;              // device staging of tps_solve_host (kept, so its graph stays valid)
+  DevBuf host_b, host_x;              // device vectors of tps_solve_host, kept
   // tps_solve_host_many: copy stream, double-buffered inputs and outputs, events
   cudaStream_t copy_stream = nullptr;
   DevBuf pipe_b[2], pipe_x[2];
@@ -724,12 +724,6 @@ void level_smooth(tps_handle *h, int level, int p, const VecLayout &lay, void *x
     smoother_sweep(h, level, p, lay, x, b, reverse, x_zero, maps, s, tc);
 }
 
-// MultigridSolvers::v_cycle (include/solver.cuh:1952-2001) on precision p:
-// input d[level], output su[level]; tc: FP32 3D sweeps on the tensor cores.
-// su[level] is zero on entry where zero_with names it: whatever writes d[level]
-// zeroes it with the same stores; otherwise it is filled here.
-// zero_init = false continues from the current su[level] instead (a further
-// cycle of v_cycle(level, n_cycles), include/solver.cuh:798-805)
 // Inside the TF32 V-cycle the tensor-core smoother runs a level only where it
 // is faster than the FP32 SIMT kernels: degrees 2..4 (the patch-GEMM kernel)
 // on levels whose colour 0 fills a wave of 128-patch tiles on every SM.
@@ -757,6 +751,12 @@ void *zero_with(const tps_handle *h, int p, int level)
   return su.bytes <= (size_t(16) << 20) ? su.p : nullptr;
 }
 
+// MultigridSolvers::v_cycle (include/solver.cuh:1952-2001) on precision p:
+// input d[level], output su[level]; tc: FP32 3D sweeps on the tensor cores.
+// su[level] is zero on entry where zero_with names it: whatever writes d[level]
+// zeroes it with the same stores; otherwise it is filled here.
+// zero_init = false continues from the current su[level] instead (a further
+// cycle of v_cycle(level, n_cycles), include/solver.cuh:798-805)
 void vcycle_rec(tps_handle *h, int level, int p, bool symmetric, cudaStream_t s, bool tc,
                 bool zero_init = true)
 {
@@ -1968,8 +1968,8 @@ int tps_solve_host_many(tps_handle *h, const tps_solve_opts *opts, int n, const 
     cudaStream_t s = h->own_stream, cs = h->copy_stream;
     // the copies stay ordered on the copy stream: H2D of b[i+1] is queued while
     // solve i runs, then D2H of x[i] once solve i is done, so both overlap solve
-    // i+1.  Every solve starts from zero in host_x (a fixed vector, so the
-    // captured CG iteration is reused) and is copied out to pipe_x.
+    // i+1.  Every solve starts from zero in host_x and is copied out to pipe_x,
+    // whose previous content may still be on its way to the host.
     try {
       TPS_CUDA(cudaMemcpyAsync(h->pipe_b[0].p, b_host[0], bytes, cudaMemcpyHostToDevice, cs));
       TPS_CUDA(cudaEventRecord(h->pipe_in[0], cs));

@@ -331,9 +331,9 @@ def test_constant_coarse_level_holds_no_workspace(cuda):
         P.close()
 
 
-# the varying-coefficient operator and smoother: tiles with remainders, several
-# layer chunks, every degree (the cells' rows are split over two thread groups
-# in FP64 from degree 5 on); padded rows are covered by the V-cycles elsewhere
+# the varying-coefficient operator: tiles with remainders, several layer chunks,
+# every degree (the smoother's are in test_gpu_kappa.py); padded rows are covered
+# by the V-cycles elsewhere
 @pytest.mark.parametrize("k,n", [(1, 9), (1, 40), (2, 3), (2, 24), (3, 5), (3, 12), (4, 2), (4, 12), (5, 3), (5, 8), (6, 2),
                                  (6, 8), (7, 2), (7, 4)])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
