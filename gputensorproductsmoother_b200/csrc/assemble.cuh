@@ -19,9 +19,10 @@
 // z stage sums the two cells of a vertex row and accumulates the column's k+1
 // z nodes in registers, the last of which opens the next layer.
 //
-// What bounds it: the latency of the two barriers per plane and FP64 issue
-// (about 45 multiply-adds per node with the halo); f is read once from HBM and
-// its halo from L2.  Measured, us, one thread per cell in 2^dim colour launches
+// What bounds it: the latency of the two barriers per plane and of the loads
+// between them at 19 warps per SM (3.1 cycles each of 12.9 per issue at Q4 48^3), then
+// the shared-memory pipe (59 % of its wavefront peak; FP64 pipe 26 %, DRAM 24 %);
+// f is read once from HBM and its halo from L2.  Measured, us, one thread per cell in 2^dim colour launches
 // / now: 3D Q4 48^3 448 / 87, Q2 96^3 292 / 108, Q5 32^3 772 / 68, Q7 16^3 4974 /
 // 70, Q4 8^3 277 / 18; 2D Q4 512^2 149 / 31, Q7 256^2 124 / 46.
 #pragma once

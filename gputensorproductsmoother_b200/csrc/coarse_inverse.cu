@@ -8,11 +8,13 @@
 // launch per block of 32 columns, out of place between two buffers: with the
 // diagonal block D, its row panel R and column panel C,
 //   A_kk <- D^-1, A_kj <- D^-1 R_j, A_ik <- -C_i D^-1, A_ij <- A_ij - C_i D^-1 R_j.
-// Every CTA inverts the 32 x 32 diagonal block itself (about 2 us, against a
-// launch of its own and its hand-over) and updates a 64 x 64 tile.
+// Every CTA inverts the 32 x 32 diagonal block itself, which saves a launch and
+// its hand-over per block, and updates a 64 x 64 tile.
 //
-// What bounds it: the chain of n / 32 launches, each one block inversion deep
-// (the matrix stays in L2).  It replaces a Cholesky inverse on the host:
+// What bounds it: the chain of n / 32 launches, each the 32 eliminations of a block
+// deep, three barriers apiece (25 to 30 us a launch up to 361 rows, 50 at 1331, where
+// three CTAs share an SM; the matrix stays in L2: DRAM 3 %, shared-memory pipe 55 %
+// of its wavefront peak).  It replaces a Cholesky inverse on the host:
 // measured for 1331 rows (a kappa update at Q4, 3^3 coarse cells) 76 ms there,
 // 2.1 ms here.
 #include "coarse_inverse.cuh"

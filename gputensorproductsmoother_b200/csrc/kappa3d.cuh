@@ -22,8 +22,9 @@
 // D^-1/2 takes 27 values per patch (a node lies below, on or above the centre
 // plane in each direction), formed by 27 threads.
 //
-// What bounds it: FP64 issue and shared-memory wavefronts (about 460
-// multiply-adds per 50 shared loads in the yz stage at degree 4).  The kernel
+// What bounds it: shared-memory wavefronts (78 % of their peak at Q4 48^3 FP64; issue
+// 57 %, FP64 pipe 37 %, 36 % of the warps by shared memory), although the yz stage
+// does about 460 multiply-adds per 50 shared loads there.  The kernel
 // before it ran the stages cell by cell with three shared-memory exchanges and
 // two square roots and divisions per node.  Measured, us per sweep on caller
 // vectors, before / now: Q4 48^3 FP64 3084 / 618, FP32 1416 / 430; Q4 12^3 FP64

@@ -12,7 +12,9 @@
 // once, to be gathered by the tile's nodes in a fixed order (deterministic, no
 // atomics); the layer's upper node plane is carried in registers.
 //
-// What bounds it: FP64 issue and its latency at 16 warps per SM; each plane is
+// What bounds it: the FP64 pipe (46 % active at Q4 48^3) and the shared-memory pipe
+// (58 % of its wavefront peak) at the 15 warps per SM that 128 registers leave,
+// which do not cover the load latency (3.1 of 7.4 cycles per issue); each plane is
 // read about 1.4 times (L2) and every dst entry written once.  It replaces 8
 // colour launches with a read-modify-write of dst each, a fill and a finishing
 // pass.  Measured, us per vmult, before / now: Q4 48^3 FP64 232 / 115, FP32 217 /

@@ -22,8 +22,10 @@
 //   -> row l (one transposition through shared memory): S^T_x, 1/lambda, S_x
 //   -> column l: S_y, store (lanes along x).
 //
-// What bounds it: the latency of these stages on small levels, instruction
-// issue on large ones.  The kernel before it held a stage's 1D lines of 4 to 16
+// What bounds it: the latency of these stages on small levels; on large ones the
+// shared-memory pipe (54 % of its wavefront peak at Q5 384^2 FP32) and the wait for
+// global loads (3.7 of 9.6 cycles per issue), with the 20 warps per SM that 85
+// registers leave (issue 48 %, DRAM 18 %).  The kernel before it held a stage's 1D lines of 4 to 16
 // patches on a CTA of 128 threads (36 busy lanes of 128 at degree 5) between
 // CTA barriers and contracted the full box.  Measured, us per sweep, before /
 // now: Q5 384^2 FP32 226 / 53, FP64 286 / 95; Q7 320^2 FP32 300 / 84, FP64 466 /

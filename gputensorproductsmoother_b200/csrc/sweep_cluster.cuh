@@ -11,9 +11,10 @@
 // the tables are constant.  The patch solves are those of the per-colour
 // kernels, operation for operation, so the sweeps are bit-identical.
 //
-// What bounds it: the latency of a patch solve and, between CTAs, of the barrier
-// and the trip through L2, 1 to 2 us a colour together, which is why only the
-// smallest levels gain (the rule and its measurements: sweep_pays).
+// What bounds it: the latency of a patch solve (the teams wait 27 of 36 cycles per
+// issue at the barriers between their stages, 3D Q4 4^3 FP32) and, between CTAs, of
+// the cluster barrier and the trip through L2, 1 to 2 us a colour together, which is
+// why only the smallest levels gain (the rule and its measurements: sweep_pays).
 //
 // 2D: warps of Sm2Lane (smoother2d.cuh).  3D: teams of threads, one line of
 // every stage per thread (the widest stage sets the team: (2k-1)(2k+1) lines),
