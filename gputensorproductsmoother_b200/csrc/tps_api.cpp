@@ -1712,7 +1712,11 @@ int tps_set_kappa(tps_handle *h, const double *kappa, int rebuild_coarse)
       build_dense_coarse(h);
       if (h->vc[1].ready) round_coarse_inverse(h);
     }
-    settings_changed(h);
+    // a batch's graph stays: every buffer that it reads was rewritten in place
+    if (h->graph) {  // re-captured on the next solve
+      cudaGraphExecDestroy(h->graph);
+      h->graph = nullptr;
+    }
   });
 }
 

@@ -102,6 +102,47 @@ def test_batch_takes_up_settings_of_its_systems(cuda):
     B.close()
 
 
+def test_batch_takes_up_new_coefficients(cuda):
+    """New coefficients of a batch's systems apply to its next solve: coarse
+    inverses formed on the host (9 rows) and on the device (125 and 512 rows)."""
+    import ctypes
+    from gputensorproductsmoother_b200 import _lib as L
+    lib, shapes = L.lib(), [(2, 2, 8, 2), (3, 2, 6, 3), (3, 3, 6, 3)]
+    rng = np.random.default_rng(12)
+    kap = [[np.exp(rng.normal(0.0, 0.4, n ** d)) for d, k, n, nc in shapes] for _ in range(2)]
+    rhs = [interior_random(d, n * k + 1, 40 + i) for i, (d, k, n, nc) in enumerate(shapes)]
+
+    def batch(kappas):
+        arr = (L.TpsProblem * len(shapes))(*[
+            L.TpsProblem(d, k, nc, (n // nc).bit_length(), 1.0, q.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), 0)
+            for (d, k, n, nc), q in zip(shapes, kappas)])
+        B = ctypes.c_void_p()
+        assert lib.tps_batch_create(arr, len(shapes), ctypes.byref(B)) == L.TPS_OK
+        return B
+
+    def solve(B, precision):
+        xs = [torch.zeros_like(v) for v in rhs]
+        o = L.TpsSolveOpts(L.DRIVER_CG, precision, 1, 100, 1e-10, 1e-300, 1)
+        reps = (L.TpsReport * len(shapes))()
+        ptrs = [(ctypes.c_void_p * len(shapes))(*[v.data_ptr() for v in vs]) for vs in (rhs, xs)]
+        assert lib.tps_batch_solve(B, ctypes.byref(o), *ptrs, reps, None) == L.TPS_OK
+        return xs, [r.iterations for r in reps]
+
+    for precision in (L.VCYCLE_F32, L.VCYCLE_F64):
+        B, C = batch(kap[0]), batch(kap[1])
+        first, _ = solve(B, precision)
+        for i in range(len(shapes)):
+            h = ctypes.c_void_p()
+            assert lib.tps_batch_system(B, i, ctypes.byref(h)) == L.TPS_OK
+            assert lib.tps_set_kappa(h, kap[1][i].ctypes.data, 1) == L.TPS_OK
+        (got, it), (want, wit) = solve(B, precision), solve(C, precision)
+        assert it == wit
+        for g, w, f in zip(got, want, first):
+            assert torch.equal(g, w) and not torch.equal(g, f)
+        lib.tps_batch_destroy(B)
+        lib.tps_batch_destroy(C)
+
+
 def test_batch_of_the_largest_number_of_systems(cuda):
     """256 systems in one graph; every one its own solution."""
     systems = [(2, 1 + i % 3, 4 + 2 * (i % 5)) for i in range(256)]
