@@ -114,6 +114,10 @@ bool injected_alloc_fault()
   return false;
 }
 
+// Gives back device memory that the handle of the running call holds only to be
+// faster (the copies of tps_smoother_step); false where there is none.
+bool give_back_copies();
+
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
@@ -131,15 +135,25 @@ struct DevBuf {
   {
     release();
     if (b == 0) return;
-    if (injected_alloc_fault())
-      throw ApiError(TPS_ERR_ALLOC, "cudaMalloc: out of memory (injected by tps_inject_alloc_failure)");
-    cudaError_t e = cudaMalloc(&p, b);
-    if (e != cudaSuccess) {
-      p = nullptr;
-      throw ApiError(TPS_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    }
+    std::string why;
+    cudaError_t e = try_alloc(b, why);
+    if (e == cudaErrorMemoryAllocation && give_back_copies()) e = try_alloc(b, why);
+    if (e != cudaSuccess) throw ApiError(TPS_ERR_ALLOC, "cudaMalloc: " + why);
     bytes = b;
     TPS_CUDA(cudaMemset(p, 0, b));
+  }
+  cudaError_t try_alloc(size_t b, std::string &why)
+  {
+    if (injected_alloc_fault()) {
+      why = "out of memory (injected by tps_inject_alloc_failure)";
+      return cudaErrorMemoryAllocation;
+    }
+    const cudaError_t e = cudaMalloc(&p, b);
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();
+    p = nullptr;
+    why = cudaGetErrorString(e);
+    return e;
   }
   void swap(DevBuf &o)
   {
@@ -282,6 +296,32 @@ void check_level(const tps_handle *h, int level, int min_level = 0)
     throw ApiError(TPS_ERR_INVALID, "level " + std::to_string(level) + " out of range");
 }
 
+// the handle whose copies an allocation of this thread may give back; null where
+// its stage_mutex is held
+thread_local tps_handle *t_running = nullptr;
+
+struct Running {
+  tps_handle *outer = t_running;
+  explicit Running(tps_handle *h) { t_running = h; }
+  Running(const Running &) = delete;
+  ~Running() { t_running = outer; }
+};
+
+bool give_back_copies()
+{
+  if (!t_running) return false;
+  tps_handle *h = t_running;
+  std::lock_guard<std::mutex> lock(h->stage_mutex);
+  bool any = false;
+  for (int p = 0; p < 2; ++p) {
+    any = any || h->stage_x[p].p || h->stage_b[p].p;
+    h->stage_maps[p].clear();  // the next sweep allocates them again
+    h->stage_x[p].release();   // (waits for the sweeps that use them)
+    h->stage_b[p].release();
+  }
+  return any;
+}
+
 template <typename F>
 int guarded(tps_handle *h, F &&f)
 {
@@ -289,6 +329,7 @@ int guarded(tps_handle *h, F &&f)
     g_create_error = "null handle";
     return TPS_ERR_INVALID;
   }
+  Running running(h);
   try {
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) throw ApiError(TPS_ERR_CUDA, cudaGetErrorString(e));
@@ -1562,6 +1603,7 @@ int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *
     const int p = dt_index(dtype);
     if (stage_pays(h, level) && !is_capturing(s)) {
       std::lock_guard<std::mutex> lock(h->stage_mutex);
+      Running none(nullptr);  // nothing is given back while the copies are in use
       if (stage_vectors(h, p)) {
         staged_smoother_step(h, level, p, x, b, zero_init != 0, reverse != 0, s);
         return;

@@ -82,7 +82,8 @@ int tps_laplace_vmult(tps_handle *h, int level, int dtype, void *dst, const void
  * reverse=1 runs the colours in reverse order (symmetric post-smoothing).
  * 3D sweeps at degree >= 3 or of at least 2e5 DoFs work on row-padded copies
  * of x and b: the first such call of a precision allocates two vectors of the
- * finest level's size, which the handle keeps.  Without memory for them, and
+ * finest level's size, which the handle keeps until another allocation of its
+ * calls would fail.  Without memory for them, and
  * inside a stream capture (whose replays may run beside other sweeps of the
  * handle), the sweep works on x and b in place; same results. */
 int tps_smoother_step(tps_handle *h, int level, int dtype, void *x, const void *b,

@@ -138,6 +138,37 @@ def test_smoother_3d_copies_with_one_stream_handle(cuda):
     P.close()
 
 
+def test_copies_are_given_back_where_memory_runs_out(cuda):
+    """Sweeps on copies take no memory from the handle's other calls: an
+    allocation that fails while the copies are held succeeds without them, and
+    sweeps go on with new ones."""
+    from gputensorproductsmoother_b200 import _lib as L
+    P, Q = tps.PoissonProblem(3, 4, 8), tps.PoissonProblem(3, 4, 8)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    b = torch.rand(P.n_dofs(), device="cuda", dtype=torch.float64, generator=gen)
+    x, y, z, w = torch.zeros_like(b), torch.zeros_like(b), torch.empty_like(b), torch.empty_like(b)
+    tps.PatchSmoother(P).step(x, b)
+    tps.PatchSmoother(Q).step(y, b)
+    tps.MultigridSolvers(Q).vmult(w, b, precision="fp64")
+    L.lib().tps_inject_alloc_failure(3)
+    try:
+        tps.MultigridSolvers(P).vmult(z, b, precision="fp64")
+    finally:
+        L.lib().tps_inject_alloc_failure(0)
+    tps.PatchSmoother(P).step(x, b)
+    tps.PatchSmoother(Q).step(y, b)
+    torch.cuda.synchronize()
+    assert torch.equal(z, w) and torch.equal(x, y)
+    # nothing left to give back: the failure is reported
+    R = tps.PoissonProblem(3, 4, 8)
+    L.lib().tps_inject_alloc_failure(3)
+    with pytest.raises(tps.TpsError):
+        tps.MultigridSolvers(R).vmult(z, b, precision="fp64")
+    L.lib().tps_inject_alloc_failure(0)
+    for p in (P, Q, R):
+        p.close()
+
+
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 def test_captured_sweeps_share_nothing(cuda, dtype):
     """Sweeps captured after the handle has its copies: two branches of one
