@@ -71,12 +71,26 @@ cudaError_t upload_one(const DegreeData &D)
       t.evec_p[r * C + q] = Pair<T>::make(t.evec[r * M + q], t.evec[r * M + C + 1 + q]);
   std::vector<LaneTables<K, T>> lane(1);  // too large for the stack at degree 7
   LaneTables<K, T> &lt = lane[0];
+  // S Lambda^-1 S^T with S rounded to T: the rounding scales mode j by a_j = s_j^T
+  // M s~_j, twice per direction, which the reciprocal eigenvalues take out again
+  // (error of a patch solve in FP32, without / with: degree 1 1.7e-7 / 0.7e-7, degree
+  // 2 1.2e-7 / 0.9e-7, degree 5 1.6e-7 / 1.4e-7)
+  double a2[M];
+  for (int j = 0; j < M; ++j) {
+    double a = 0.0;
+    for (int r = 0; r < M; ++r)
+      for (int q = 0; q < M; ++q)
+        a += D.evec[r * M + j] * D.pmass[(r + 1) * N1 + q + 1] * static_cast<double>(t.evec[q * M + j]);
+    a2[j] = a * a;
+  }
   for (int z = 0; z < M; ++z)
     for (int y = 0; y < M; ++y)
       for (int x = 0; x < M; ++x)
-        lt.rlam3[(z * M + y) * M + x] = static_cast<T>(1.0 / (D.eval[x] + D.eval[y] + D.eval[z]));
+        lt.rlam3[(z * M + y) * M + x] =
+            static_cast<T>(1.0 / ((D.eval[x] + D.eval[y] + D.eval[z]) * (a2[x] * a2[y] * a2[z])));
   for (int y = 0; y < M; ++y)
-    for (int x = 0; x < M; ++x) lt.rlam2[y * M + x] = static_cast<T>(1.0 / (D.eval[y] + D.eval[x]));
+    for (int x = 0; x < M; ++x)
+      lt.rlam2[y * M + x] = static_cast<T>(1.0 / ((D.eval[y] + D.eval[x]) * (a2[y] * a2[x])));
   for (int j = 0; j < N1; ++j)
     for (int r = 0; r < M; ++r) {
       lt.prows2[j * M + r] = static_cast<T>(D.pmass[(r + 1) * N1 + j]);

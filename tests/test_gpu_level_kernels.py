@@ -43,6 +43,26 @@ def test_smoother_2d_launch_shapes(cuda, oracle, k, n, dtype):
     sweep_matches(oracle, 2, k, n, dtype, relaxation=0.9)
 
 
+# A patch solve in FP32 rounds each of its stages and its result once, and its
+# tables once: independent errors of at most 2^-24 each, of which the last ones
+# count fully and the stages' average out.  Against the FP64 sweep they stay below
+# three units in the 2-norm; one factor common to all entries (the rounding of a
+# mode's length, left in) takes more than that by itself at degree 1.
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 6, 7])
+def test_smoother_2d_fp32_rounding(cuda, k):
+    for n in (12, 48, 96):
+        P = tps.PoissonProblem(2, k, n)
+        S = tps.PatchSmoother(P)
+        gen = torch.Generator(device="cuda").manual_seed(100 * k + n)
+        x, b = (torch.rand(P.n_dofs(), device="cuda", generator=gen) * 2 - 1 for _ in range(2))
+        x64 = x.double()
+        S.step(x, b)
+        S.step(x64, b.double())
+        torch.cuda.synchronize()
+        assert ((x.double() - x64).norm() / x64.norm()).item() < 3 * 2.0 ** -24
+        P.close()
+
+
 # the sweep on row-padded copies of the caller's vectors: one and several
 # levels sharing the copies, the smallest level that takes them, rows that
 # need 0..3 entries of padding
