@@ -401,8 +401,8 @@ std::vector<double> dense_coarse_host(const tps_handle *h)
 }
 
 // the same on the device, into the handle's inverse, which is replaced once the
-// new one is known to be good
-void dense_coarse_device(tps_handle *h, int ni)
+// new one is known to be good; false where a pivot is not positive
+bool dense_coarse_device(tps_handle *h, int ni)
 {
   const int k = h->k, n = h->n_coarse, dim = h->dim;
   const size_t n2 = static_cast<size_t>(ni) * ni, nt = h->D.cmass.size();
@@ -421,7 +421,7 @@ void dense_coarse_device(tps_handle *h, int ni)
   TPS_CUDA(launch_spd_inverse(a, a + n2, ni, bad, nullptr));
   int failed = 0;
   TPS_CUDA(cudaMemcpy(&failed, bad, sizeof(int), cudaMemcpyDeviceToHost));
-  if (failed) throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
+  if (failed) return false;
   TPS_CUDA(cudaMemcpyAsync(first.p ? first.p : h->coarse_inv.p, a, sizeof(double) * n2, cudaMemcpyDeviceToDevice,
                            nullptr));
   TPS_CUDA(cudaStreamSynchronize(nullptr));  // any stream may read it from here on
@@ -429,6 +429,8 @@ void dense_coarse_device(tps_handle *h, int ni)
   // kept for the updates of a coefficient, which then cannot run out of memory
   // half-way; a constant one is inverted once
   if (!h->has_kappa) h->coarse_work.release();
+  h->coarse_inv_host.clear();
+  return true;
 }
 
 // A small coarse operator is inverted on the host, a larger one on the device.
@@ -443,13 +445,13 @@ void build_dense_coarse(tps_handle *h)
 {
   const int m1 = h->n_coarse * h->k - 1, dim = h->dim;
   const int ni = dim == 3 ? m1 * m1 * m1 : m1 * m1;
-  if (ni <= (h->has_kappa ? 110 : 200)) {
+  // coefficients over 1e30 and more can lose definiteness to rounding; the host's
+  // Cholesky then has the last word
+  if (ni <= (h->has_kappa ? 110 : 200) || !dense_coarse_device(h, ni)) {
     h->coarse_inv_host = dense_coarse_host(h);
     if (h->coarse_inv.p)
       TPS_CUDA(cudaMemcpy(h->coarse_inv.p, h->coarse_inv_host.data(), sizeof(double) * h->coarse_inv_host.size(),
                           cudaMemcpyHostToDevice));
-  } else {
-    dense_coarse_device(h, ni);
   }
   h->n_int_coarse = ni;
   h->coarse_coord.resize(3 * static_cast<size_t>(ni));
@@ -464,8 +466,8 @@ void build_dense_coarse(tps_handle *h)
 void coarse_inverse_on_device(tps_handle *h)
 {
   if (h->coarse_inv.p) return;
-  if (h->coarse_inv_host.empty()) {
-    dense_coarse_device(h, h->n_int_coarse);
+  if (h->coarse_inv_host.empty()) {  // a constant coefficient's, released by FP32 V-cycles
+    if (!dense_coarse_device(h, h->n_int_coarse)) throw ApiError(TPS_ERR_INVALID, "coarse operator not positive definite");
     return;
   }
   DevBuf inv;

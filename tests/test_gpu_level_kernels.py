@@ -324,6 +324,27 @@ def test_dense_coarse_inverse(cuda, dim, k, n, varying):
     P.close()
 
 
+def test_coefficients_at_the_limit_of_definiteness(cuda):
+    """Coefficients over 1e30: where the device's elimination meets a pivot that
+    rounding made negative, the host's factorisation decides, as it does for
+    small coarse levels."""
+    for seed in range(5):
+        kap = np.exp(np.random.default_rng(seed).normal(0.0, 15.0, (2, 17 ** 2)))
+        P = tps.PoissonProblem(2, 1, 17, n_coarse=17, kappa=kap[0])
+        b = torch.rand(P.n_dofs(), dtype=torch.float64, device="cuda")
+        z = P.new_vector()
+        tps.MultigridSolvers(P).vmult(z, b, precision="fp64")
+        P.set_kappa(np.ones(17 ** 2))  # a definite one afterwards is that of a new handle
+        Q = tps.PoissonProblem(2, 1, 17, n_coarse=17, kappa=np.ones(17 ** 2))
+        w = P.new_vector()
+        tps.MultigridSolvers(P).vmult(z, b, precision="fp64")
+        tps.MultigridSolvers(Q).vmult(w, b, precision="fp64")
+        torch.cuda.synchronize()
+        assert torch.equal(z, w)
+        P.close()
+        Q.close()
+
+
 def test_kappa_update_needs_no_memory(cuda):
     """A new coefficient is taken up whole where device memory has run out, also
     with a large dense coarse level (2601 rows, 54 MB a matrix)."""
